@@ -20,7 +20,7 @@ int pcg_block_size();
 void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks = 0);
 int pcg_check_structured(const LevelDev &F, const LevelDev &C);
 float *pcg_build_rw16(const LevelDev &F, const LevelDev &C);
-float *pcg_dense_map(const SolveParams &prm, int l0, int ld);
+double *pcg_dense_map(const SolveParams &prm, int l0);
 
 constexpr int kB = 256;
 
@@ -398,8 +398,8 @@ struct FluidPriv {
     unsigned int *vmax_host = nullptr;
     int structured[kMaxLev] = {};  // level l -> l+1 transfers follow the index pattern
     float *rw16[kMaxLev] = {};     // coarse-major structured restriction weights
-    float *dense = nullptr;        // dense map of the V-cycle below the grid levels
-    int nd = 0, ld = 0;
+    double *dense = nullptr;       // dense map of the V-cycle below the grid levels
+    int nd = 0;
     int last_flags = 0;            // kSolve* bits of the last solve
     // mixed-precision solve (ggb_fluid_set_precision): FP16 level vectors,
     // FP16 slot weights of the coarse levels, the previous z
@@ -483,12 +483,6 @@ static void build_levels(Fluid *F, FluidPriv *Pv) {
 }
 
 constexpr int kBlockLevelMax = 1536;  // levels up to N=16 form the dense coarse map
-// A coarsest level of more cells (grids whose edge halves only to an odd
-// number above 16) also becomes a dense map up to this many cells (N = 32):
-// its 60 Jacobi sweeps, each with a grid barrier, take 250 us per V-cycle at
-// N = 25 against 13 us for reading that map's 56 MB.  At 6144 cells the map
-// takes 151 MB, more than L2 holds, and four times as much at twice the cells.
-constexpr int kDenseMax = 6144;
 
 static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int maxit) {
     if (F->cs->N > pcg_max_grid_n())
@@ -534,10 +528,10 @@ static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int ma
         while (G < Pv->nlev - 1 && P.L[G].S.n > kBlockLevelMax) G++;
         if (G < 1) G = 1;
         P.nlev_grid = G;
-        P.coarse_on_grid = (G == Pv->nlev - 1 && P.L[Pv->nlev - 1].S.n > kDenseMax) ? 1 : 0;
+        P.coarse_on_grid = (G == Pv->nlev - 1 && P.L[Pv->nlev - 1].S.n > kBlockLevelMax) ? 1 : 0;
     } else if (mg) {
         P.nlev_grid = 0;
-        P.coarse_on_grid = P.L[0].S.n > kDenseMax ? 1 : 0;
+        P.coarse_on_grid = P.L[0].S.n > kBlockLevelMax ? 1 : 0;
     }
     P.area = F->cs->area;
     P.omega = F->omega;
@@ -556,7 +550,6 @@ static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int ma
     if (mg && Pv->dense) {
         P.dense = Pv->dense;
         P.nd = Pv->nd;
-        P.ld = Pv->ld;
     }
     return P;
 }
@@ -571,11 +564,13 @@ static void finish_levels(Fluid *F, FluidPriv *Pv) {
         Pv->structured[l] = pcg_check_structured(Fl, C);
         if (Pv->structured[l]) Pv->rw16[l] = pcg_build_rw16(Fl, C);
     }
-    P = solve_params(F, Pv, 0, 1);  // with the structured flags
-    if (!P.coarse_on_grid) {
-        Pv->nd = P.L[P.nlev_grid].S.n;
-        Pv->ld = (Pv->nd + 3) & ~3;
-        Pv->dense = pcg_dense_map(P, P.nlev_grid, Pv->ld);
+    if (Pv->nlev >= 2) {
+        P = solve_params(F, Pv, 0, 1);  // with the structured flags
+        int G = P.nlev_grid;
+        if (G < Pv->nlev && P.L[G].S.n <= kBlockLevelMax) {
+            Pv->dense = pcg_dense_map(P, G);
+            Pv->nd = P.L[G].S.n;
+        }
     }
 }
 

@@ -65,8 +65,8 @@ struct SolveParams {
     GridBarrier *bar;
     SolveResult *res;
     // dense form of the V-cycle below the grid levels: xo_G = D b_G
-    const float *dense;  // [nd][ld] row-major (rows padded with zeros to ld), or nullptr
-    int nd, ld;          // cells of level nlev_grid; row stride, a multiple of 4
+    const double *dense;  // [nd][nd] row-major, or nullptr
+    int nd;               // cells of level nlev_grid
 };
 
 }  // namespace ggb

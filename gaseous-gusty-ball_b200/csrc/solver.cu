@@ -69,8 +69,8 @@ __global__ void __launch_bounds__(kPB, 1) k_pcg_batch(const SolveParams *prm, co
 // ---- setup kernels -------------------------------------------------------
 
 // Column j of the dense map of levels l0..nlev-1: the block's V-cycle applied
-// to the unit vector e_j, stored row-major D[row][j] (row stride ld).
-__global__ void __launch_bounds__(kPB, 1) k_dense_columns(SolveParams P, int l0, float *D, int ld) {
+// to the unit vector e_j, stored row-major D[row][j] in FP64.
+__global__ void __launch_bounds__(kPB, 1) k_dense_columns(SolveParams P, int l0, double *D) {
     extern __shared__ __align__(16) unsigned char dyn[];
     float *smem = reinterpret_cast<float *>(dyn);
     const int nd = P.L[l0].S.n;
@@ -80,74 +80,7 @@ __global__ void __launch_bounds__(kPB, 1) k_dense_columns(SolveParams P, int l0,
         BLOCK_LOOP(c, nd) lv[l0].b[c] = c == j ? 1.0f : 0.0f;
         __syncthreads();
         vcycle_block_smem(P, l0, lv);
-        BLOCK_LOOP(c, nd) D[(size_t)c * ld + j] = lv[l0].xo[c];
-        __syncthreads();
-    }
-}
-
-// The links of every cell of a level as [8][n] neighbour indices and weights
-// (unused links: the cell itself with weight 0).
-__global__ void k_links(StencilDev S, unsigned short *nb, float *w) {
-    KERNEL_LOOP(c, S.n) {
-        int o[kMaxNb];
-        float q[kMaxNb];
-        cell_links(S, c, o, q);
-        for (int k = 0; k < kMaxNb; k++) {
-            nb[(size_t)k * S.n + c] = (unsigned short)o[k];
-            w[(size_t)k * S.n + c] = q[k];
-        }
-    }
-}
-
-// Columns of the dense map of one level that is only swept (coarsest_smem's
-// arithmetic): four unit vectors at a time as the components of float4 vectors
-// in shared memory, so that a cell's links are read once for four columns.
-// Bound by the FP64 conversions (one per neighbour value).  One column per
-// block and pass, its links through the slot tables, took 21 ms at nd = 3750.
-constexpr int kSweepThreads = 1024;
-__global__ void __launch_bounds__(kSweepThreads, 1)
-    k_dense_sweeps(int n, const unsigned short *nb, const float *w, const float *dinv, int sweeps, float *D, int ld) {
-    extern __shared__ __align__(16) unsigned char dyn[];
-    float4 *src = reinterpret_cast<float4 *>(dyn), *dst = src + n;
-    for (int j = 4 * blockIdx.x; j < n; j += 4 * gridDim.x) {
-        BLOCK_LOOP(c, n) src[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncthreads();
-        for (int s = 0; s < sweeps; s++) {
-            BLOCK_LOOP(c, n) {
-                const float4 xc = src[c];
-                const double xx = xc.x, xy = xc.y, xz = xc.z, xw = xc.w;
-                double ax = 0, ay = 0, az = 0, aw = 0;
-#pragma unroll
-                for (int k = 0; k < kMaxNb; k++) {
-                    const float4 v = src[__ldg(nb + (size_t)k * n + c)];
-                    const double q = __ldg(w + (size_t)k * n + c);
-                    ax += q * (xx - (double)v.x);
-                    ay += q * (xy - (double)v.y);
-                    az += q * (xz - (double)v.z);
-                    aw += q * (xw - (double)v.w);
-                }
-                const double om = kOmegaJ * __ldg(dinv + c);
-                const int u = c - j;
-                float4 o;
-                o.x = xc.x + (float)(om * (float)((u == 0 ? 1.0f : 0.0f) - ax));
-                o.y = xc.y + (float)(om * (float)((u == 1 ? 1.0f : 0.0f) - ay));
-                o.z = xc.z + (float)(om * (float)((u == 2 ? 1.0f : 0.0f) - az));
-                o.w = xc.w + (float)(om * (float)((u == 3 ? 1.0f : 0.0f) - aw));
-                dst[c] = o;
-            }
-            __syncthreads();
-            float4 *t = src;
-            src = dst;
-            dst = t;
-        }
-        // ld is a multiple of 4: past the last column a row holds padding, kept 0
-        BLOCK_LOOP(c, n) {
-            float4 o = src[c];
-            if (j + 1 >= n) o.y = 0.f;
-            if (j + 2 >= n) o.z = 0.f;
-            if (j + 3 >= n) o.w = 0.f;
-            *reinterpret_cast<float4 *>(D + (size_t)c * ld + j) = o;
-        }
+        BLOCK_LOOP(c, nd) D[(size_t)c * nd + j] = lv[l0].xo[c];
         __syncthreads();
     }
 }
@@ -216,7 +149,7 @@ static size_t pcg_smem_bytes(const SolveParams &p) {
     size_t cells = 0;
     if (p.nlev >= 2 && !p.dense && !p.coarse_on_grid)
         for (int l = p.nlev_grid; l < p.nlev; l++) cells += p.L[l].S.n;
-    if (p.nlev == 1 && !p.dense && !p.coarse_on_grid) cells = p.L[0].S.n;
+    if (p.nlev == 1 && !p.coarse_on_grid) cells = p.L[0].S.n;
     return kStageBytes + 4 * sizeof(float) * cells;
 }
 
@@ -353,36 +286,17 @@ int pcg_check_structured(const LevelDev &F, const LevelDev &C) {
     return hb == 0;
 }
 
-// The dense map of the V-cycle of levels l0..nlev-1 (nd rows of stride ld).
-float *pcg_dense_map(const SolveParams &prm, int l0, int ld) {
+// The dense map of the V-cycle of levels l0..nlev-1 (nd x nd, FP64).
+double *pcg_dense_map(const SolveParams &prm, int l0) {
     SolveParams p = prm;
     const int nd = p.L[l0].S.n;
-    float *D = (float *)dev_alloc(sizeof(float) * (size_t)nd * ld);
-    if (l0 == p.nlev - 1) {  // one level: the sweeps alone
-        unsigned short *nb = (unsigned short *)dev_alloc(sizeof(unsigned short) * kMaxNb * nd);
-        float *w = (float *)dev_alloc(sizeof(float) * kMaxNb * nd);
-        const size_t smem = 2 * sizeof(float4) * (size_t)nd;
-        static bool attr = false;
-        if (!attr) {
-            GGB_CHECK(cudaFuncSetAttribute(k_dense_sweeps, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            attr = true;
-        }
-        k_links<<<grid_for(nd, 256), 256, 0, stream()>>>(p.L[l0].S, nb, w);
-        GGB_LAUNCHED();
-        k_dense_sweeps<<<std::min((nd + 3) / 4, device_sm_count()), kSweepThreads, smem, stream()>>>(
-            nd, nb, w, p.L[l0].dinv, p.coarse_sweeps, D, ld);
-        GGB_LAUNCHED();
-        GGB_CHECK(cudaStreamSynchronize(stream()));
-        dev_free(nb);
-        dev_free(w);
-        return D;
-    }
     size_t cells = 0;
     for (int l = l0; l < p.nlev; l++) cells += p.L[l].S.n;
     size_t smem = 4 * sizeof(float) * cells;
     pcg_attributes();
     int grid = std::min(nd, 4 * device_sm_count());
-    k_dense_columns<<<grid, kPB, smem, stream()>>>(p, l0, D, ld);
+    double *D = (double *)dev_alloc(sizeof(double) * nd * nd);
+    k_dense_columns<<<grid, kPB, smem, stream()>>>(p, l0, D);
     GGB_LAUNCHED();
     GGB_CHECK(cudaStreamSynchronize(stream()));
     return D;

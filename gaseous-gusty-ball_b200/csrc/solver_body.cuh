@@ -605,35 +605,6 @@ __device__ __forceinline__ void vcycle_block_smem(const SolveParams &P, int l0, 
     }
 }
 
-// ---- the dense map ----------------------------------------------------------
-
-// put(row, sum_j D[row][j] get(j)) for every row of the dense map, one warp
-// per row, FP64 sums.  Bound by reading D from L2 (9.4 MB at nd = 1536, 56 MB
-// at 3750): 16-byte loads, four in flight per lane.  D holds FP32 values (the
-// V-cycle it was built from works on FP32 vectors), so FP32 storage loses
-// nothing against FP64 and halves the bytes.
-template <class Get, class Put>
-__device__ __forceinline__ void dense_rows(const SolveParams &P, Get get, Put put) {
-    const int nd = P.nd, ld4 = P.ld >> 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gw = vb() * (blockDim.x >> 5) + warp, nw = vnb() * (blockDim.x >> 5);
-    for (int row = gw; row < nd; row += nw) {
-        const float4 *d = reinterpret_cast<const float4 *>(P.dense) + (size_t)row * ld4;
-        double acc = 0;
-#pragma unroll 4
-        for (int j = lane; j < ld4; j += 32) {
-            const float4 w = __ldg(d + j);
-            const int k = 4 * j;
-            acc += (double)w.x * (double)get(k);
-            acc += (double)w.y * (double)get(min(k + 1, nd - 1));  // past the row's end the weight is 0
-            acc += (double)w.z * (double)get(min(k + 2, nd - 1));
-            acc += (double)w.w * (double)get(min(k + 3, nd - 1));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) put(row, acc);
-    }
-}
-
 // ---- the V-cycle after level 0's pre-smooth --------------------------------
 
 // The rest of z = V(r) once level 0's pre-smooth (x, r of level 0) is complete
@@ -660,7 +631,16 @@ __device__ bool vcycle_rest(const SolveParams &P, const float *r, float s0, floa
         const LevelDev &C = P.L[G];
         const auto *cb = lv<MP>(C.b);
         auto *cx = lv<MP>(C.xo);
-        dense_rows(P, [&](int j) { return ldv(cb, j); }, [&](int row, double v) { stv(cx, row, (float)v); });
+        const int nd = P.nd, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int gw = vb() * (blockDim.x >> 5) + warp, nw = vnb() * (blockDim.x >> 5);
+        for (int row = gw; row < nd; row += nw) {
+            const double *d = P.dense + (size_t)row * nd;
+            double acc = 0;
+            for (int j = lane; j < nd; j += 32) acc += __ldg(d + j) * (double)ldv(cb, j);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) stv(cx, row, (float)acc);
+        }
         trace_mark(P, 500);
         SYNC_OR(return false);
     } else if (!P.coarse_on_grid) {
@@ -724,9 +704,15 @@ __device__ bool single_level(const SolveParams &P, const float *r, float s0, flo
     const LevelDev &L = P.L[0];
     auto *lx = lv<MP>(L.x), *lxo = lv<MP>(L.xo);
     auto *lb = lv<MP>(L.b);
-    if (P.dense) {
-        dense_rows(P, [&](int j) { return MP ? r[j] * s0 : r[j]; },
-                   [&](int row, double v) { stv(lxo, row, (float)v); });
+    if (!P.coarse_on_grid) {
+        if (vb() == 0) {
+            SmemLevel lvs[kMaxLev];
+            carve_smem(P, 0, smem, lvs);
+            BLOCK_LOOP(c, L.S.n) lvs[0].b[c] = r[c];
+            __syncthreads();
+            coarsest_smem(L, lvs[0], P.coarse_sweeps);
+            BLOCK_LOOP(c, L.S.n) stv(lxo, c, MP ? lvs[0].xo[c] * s0 : lvs[0].xo[c]);
+        }
     } else {
         GRID_LOOP(c, L.S.n) {
             stv(lx, c, 0.f);
