@@ -524,6 +524,10 @@ struct TileSmem {
     union {
         unsigned short ent[kEnt];                 // entry lists packed by a count scan
         unsigned short bucket[kT * kT * kBucketStride];  // kBucket entry slots per texel (one-pass path)
+        struct {
+            unsigned long long key[(kRec + 31) / 32 * 32];  // runs of 32 sorted keys (composite_sorted)
+            unsigned short order[kRec];
+        } w;
     };
     int cnt[kT * kT];
     int start[kT * kT];
@@ -695,13 +699,97 @@ __device__ __forceinline__ void composite_window(TileSmem &S, int nw, const Spla
     __syncthreads();
 }
 
+// The window's records 0..m-1 (m <= kRec) composited without per-texel lists:
+// ranked by key, then walked in that order by every warp, 32 at a time, a ballot
+// leaving the records whose box meets the warp's 8 x 4 texels (wide_texel).
+// For wide splats, whose boxes hold many texels each: per (record, texel) entry
+// the lists cost a slot, an atomic and an insertion-sort step, this only the
+// blend, and a window holds any number of entries (the lists' 1728 overflow at
+// about 90 records of radius 2.5, and every window then costs two passes over the
+// tile's records).  Bound by issue: the runs and searches take about a third, the
+// walk the rest.  200k particles on 600 x 600 faces, radius 2.5: k_rd_tiles 250 us
+// against the lists' 706; ranking by counting over all records took 330.
+// The line between lists and sorted records, whole deposits in us: 300k particles
+// on 600 x 600 faces, radius 1: 144 / 179; 1.25: 173 / 190; 1.5: 209 / 200; 20k on
+// 1000 x 1000, radius 1.5: 155 / 152; 3: 219 / 166.
+constexpr float kWideRadius = 1.4f;
+__device__ __forceinline__ int wide_texel_x() { return (threadIdx.x >> 5 & 1) * 8 + (threadIdx.x & 7); }
+__device__ __forceinline__ int wide_texel_y() { return (threadIdx.x >> 6) * 4 + (threadIdx.x >> 3 & 3); }
+__device__ __forceinline__ void composite_sorted(TileSmem &S, int m, const SplatCfg &C, const TileGeo &G, float4 &d) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned short *order = S.w.order;
+    const int runs = (m + 31) >> 5;
+    __syncthreads();
+    // each warp sorts runs of 32 records by counting within the run; a record's
+    // rank is then its place in its run plus the smaller keys of every other run
+    for (int run = warp; run < runs; run += kTB / 32) {
+        const int s = run * 32 + lane;
+        const unsigned long long key = s < m ? S.u.r.key[s] : ~0ull;
+        int place = 0;
+#pragma unroll 8
+        for (int t = 0; t < 32; t++) {
+            const unsigned long long k = run * 32 + t < m ? S.u.r.key[run * 32 + t] : ~0ull;
+            place += k < key || (k == key && t < lane);
+        }
+        S.w.key[run * 32 + place] = key;
+    }
+    __syncthreads();
+    for (int s = threadIdx.x; s < m; s += kTB) {
+        const unsigned long long key = S.u.r.key[s];
+        int rank = 0;
+#pragma unroll 4
+        for (int run = 0; run < runs; run++) {
+            const unsigned long long *k = S.w.key + run * 32;
+            int at = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (k[at + step - 1] < key) at += step;
+            rank += at + (k[at] < key);
+        }
+        order[rank] = (unsigned short)s;
+    }
+    __syncthreads();
+    const int x = wide_texel_x(), y = wide_texel_y(), xw = x & 8, yw = y & 12;
+    const float invrad = C.invrad, invg = C.invg;
+    const float xf = (float)(G.x0 + x), yf = (float)(G.y0 + y);
+    for (int b = 0; b < m; b += 32) {
+        int s = 0;
+        bool hit = false;
+        if (b + lane < m) {
+            s = order[b + lane];
+            const unsigned box = S.box[s];
+            const int xa = box & 15, ya = box >> 4 & 15, xb = xa + (int)(box >> 8 & 15), yb = ya + (int)(box >> 12);
+            hit = box != kNoBox && xa <= xw + 7 && xb >= xw && ya <= yw + 3 && yb >= yw;
+        }
+        for (unsigned left = __ballot_sync(0xffffffffu, hit); left; left &= left - 1) {
+            const int sj = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+            const unsigned box = S.box[sj];
+            if ((unsigned)(x - (int)(box & 15)) > (box >> 8 & 15) || (unsigned)(y - (int)(box >> 4 & 15)) > box >> 12)
+                continue;
+            const float2 pp = S.u.r.pos[sj];
+            const float4 c = S.col[sj];
+            const float w0 = C.alpha * c.w;
+            const float wy = __fmaf_rn(-fabsf(yf - pp.y), invrad, 1.0f);
+            const float wx = __fmaf_rn(-fabsf(xf - pp.x), invrad, 1.0f);
+            const float w = __fmul_rn(__fmul_rn(w0, wx), wy);
+            const float keep = 1.0f - w, add = __fmul_rn(w, invg);
+            d.x = __fmaf_rn(d.x, keep, __fmul_rn(add, c.x));
+            d.y = __fmaf_rn(d.y, keep, __fmul_rn(add, c.y));
+            d.z = __fmaf_rn(d.z, keep, __fmul_rn(add, c.z));
+            d.w = __fmaf_rn(d.w, keep, add);
+        }
+    }
+}
+
 // A tile whose records do not fit one window: consecutive key ranges [lo, hi),
 // each holding at most kRec records and kEnt entries, composited in turn.  hi
 // is the end of the longest run of key buckets (a histogram over [lo, top])
 // within both limits; when the first bucket alone is over, the search narrows
 // to that bucket.  One key is one record (a sample falls on a tile once), and
 // a record has at most 256 entries (its box lies on the tile), so every window
-// makes progress.
+// makes progress.  WIDE windows are composited by composite_sorted and have no
+// limit on their entries.
+template <bool WIDE>
 __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col, int m, const SplatCfg &C,
                                    const TileGeo &G, float4 &d) {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -738,7 +826,7 @@ __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col,
                 const Rec r = R[s];
                 if (r.key < lo || r.key > top) continue;
                 const int e = box_entries(rec_box(C, G, r.px, r.py));
-                if (e) atomicAdd(&S.u.hist[(r.key - lo) / bw], ((unsigned long long)e << 32) | 1ull);
+                if (e) atomicAdd(&S.u.hist[(r.key - lo) / bw], ((unsigned long long)(WIDE ? 0 : e) << 32) | 1ull);
             }
             __syncthreads();
             // first bucket at which the running totals pass a limit
@@ -778,7 +866,12 @@ __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col,
         const int nw = min(S.cut, kRec);
         window_colours(S, nw, col);
         __syncthreads();
-        composite_window(S, nw, C, G, d);
+        if (WIDE) {
+            composite_sorted(S, nw, C, G, d);
+            __syncthreads();
+        } else {
+            composite_window(S, nw, C, G, d);
+        }
         lo = hi;
     }
 }
@@ -786,7 +879,9 @@ __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col,
 // One block per tile; see the file comment.  Seven blocks per SM (32
 // registers, 30.2 KB of shared memory with a 576-record window) ran 6 % faster
 // than six (40 registers, 768 records) and eight (448 records) did.
-__global__ void __launch_bounds__(kTB, 7) k_rd_tiles(SplatCfg C, const unsigned *tile_start,
+// WIDE (splat radius over kWideRadius): no per-texel lists, composite_sorted.
+template <bool WIDE>
+__global__ void __launch_bounds__(kTB, WIDE ? 6 : 7) k_rd_tiles(SplatCfg C, const unsigned *tile_start,
                                                   const unsigned *tile_fill, const Rec *recs, size_t cap,
                                                   const float4 *col, float *buf, unsigned *diag,
                                                   unsigned *est_next) {
@@ -804,7 +899,7 @@ __global__ void __launch_bounds__(kTB, 7) k_rd_tiles(SplatCfg C, const unsigned 
     G.tw = min(kT, R - G.x0);
     G.th = min(kT, R - G.y0);
     float4 *face = reinterpret_cast<float4 *>(buf) + (size_t)f * R * R;
-    const int lx = q % kT, ly = q / kT;
+    const int lx = WIDE ? wide_texel_x() : q % kT, ly = WIDE ? wide_texel_y() : q / kT;
     const bool inside = lx < G.tw && ly < G.th;
     // the texel is requested together with the tile's record count (before
     // knowing whether the tile has records), so that the two round trips
@@ -823,57 +918,71 @@ __global__ void __launch_bounds__(kTB, 7) k_rd_tiles(SplatCfg C, const unsigned 
     }
     if (m > 0) {
         const Rec *Rt = recs + s0;
-        // one window: records, per-texel counts and, while no texel takes more
-        // than kBucket entries, the entries themselves (each in the slot its
-        // count gives it) in one pass
-        S.cnt[q] = 0;
-        if (q == 0) {
-            S.tot = 0;
-            S.full = 0;
-        }
-        __syncthreads();
-        if (m <= kRec) {
-            int e = 0;
-            for (int s = q; s < m; s += kTB) {
-                const Rec r = Rt[s];
-                const unsigned short box = rec_box(C, G, r.px, r.py);
-                window_put(S, s, r, box);
-                box_texels(box, [&](int t) {
-                    const int k = atomicAdd(&S.cnt[t], 1);
-                    if (k < kBucket)
-                        S.bucket[t * kBucketStride + k] = (unsigned short)s;
-                    else
-                        S.full = 1;
-                });
-                e += box_entries(box);
+        if (WIDE) {
+            if (m <= kRec) {
+                for (int s = q; s < m; s += kTB) {
+                    const Rec r = Rt[s];
+                    window_put(S, s, r, rec_box(C, G, r.px, r.py));
+                }
+                window_colours(S, m, col);
+                composite_sorted(S, m, C, G, d);
+            } else {
+                if (q == 0) atomicAdd(diag, 1u);
+                composite_windowed<true>(S, Rt, col, m, C, G, d);
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-            if ((q & 31) == 0 && e) atomicAdd(&S.tot, e);
-            window_colours(S, m, col);  // each thread reads back the keys it stored itself
-        }
-        __syncthreads();
-        if (m <= kRec && !S.full) {
-            const int c = S.cnt[q];
-            if (c) blend_texel(S, S.bucket + q * kBucketStride, c, q, C, G, d);
-        } else if (m <= kRec && S.tot <= kEnt) {
-            // a texel with more than kBucket entries: pack the lists by a count scan
-            const int c = S.cnt[q];
-            const int st = block_scan_1sync(c, S.wsum);
-            S.start[q] = st;
-            S.cnt[q] = 0;
-            __syncthreads();
-            for (int s = q; s < m; s += kTB)
-                box_texels(S.box[s], [&](int t) {
-                    const int e = S.start[t] + atomicAdd(&S.cnt[t], 1);
-                    if (e < kEnt) S.ent[e] = (unsigned short)s;
-                });
-            __syncthreads();
-            if (c) blend_texel(S, S.ent + st, c, q, C, G, d);
         } else {
-            if (q == 0) atomicAdd(diag, 1u);
+            // one window: records, per-texel counts and, while no texel takes more
+            // than kBucket entries, the entries themselves (each in the slot its
+            // count gives it) in one pass
+            S.cnt[q] = 0;
+            if (q == 0) {
+                S.tot = 0;
+                S.full = 0;
+            }
             __syncthreads();
-            composite_windowed(S, Rt, col, m, C, G, d);
+            if (m <= kRec) {
+                int e = 0;
+                for (int s = q; s < m; s += kTB) {
+                    const Rec r = Rt[s];
+                    const unsigned short box = rec_box(C, G, r.px, r.py);
+                    window_put(S, s, r, box);
+                    box_texels(box, [&](int t) {
+                        const int k = atomicAdd(&S.cnt[t], 1);
+                        if (k < kBucket)
+                            S.bucket[t * kBucketStride + k] = (unsigned short)s;
+                        else
+                            S.full = 1;
+                    });
+                    e += box_entries(box);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+                if ((q & 31) == 0 && e) atomicAdd(&S.tot, e);
+                window_colours(S, m, col);  // each thread reads back the keys it stored itself
+            }
+            __syncthreads();
+            if (m <= kRec && !S.full) {
+                const int c = S.cnt[q];
+                if (c) blend_texel(S, S.bucket + q * kBucketStride, c, q, C, G, d);
+            } else if (m <= kRec && S.tot <= kEnt) {
+                // a texel with more than kBucket entries: pack the lists by a count scan
+                const int c = S.cnt[q];
+                const int st = block_scan_1sync(c, S.wsum);
+                S.start[q] = st;
+                S.cnt[q] = 0;
+                __syncthreads();
+                for (int s = q; s < m; s += kTB)
+                    box_texels(S.box[s], [&](int t) {
+                        const int e = S.start[t] + atomicAdd(&S.cnt[t], 1);
+                        if (e < kEnt) S.ent[e] = (unsigned short)s;
+                    });
+                __syncthreads();
+                if (c) blend_texel(S, S.ent + st, c, q, C, G, d);
+            } else {
+                if (q == 0) atomicAdd(diag, 1u);
+                __syncthreads();
+                composite_windowed<false>(S, Rt, col, m, C, G, d);
+            }
         }
     }
     if (inside) face[(size_t)(G.y0 + ly) * R + G.x0 + lx] = d;
@@ -932,8 +1041,9 @@ static void deposit_fill_tiles(Render *r, const Particles *P, RenderPriv *Pv, co
                                      Pv->rec_cap, Pv->diag);
         GGB_LAUNCHED();
     }
-    k_rd_tiles<<<Pv->ntiles, kTB, 0, s>>>(C, Pv->tile_start, Pv->tile_fill, Pv->recs, Pv->rec_cap,
-                                          reinterpret_cast<const float4 *>(P->col), r->buf, Pv->diag, Pv->tile_est);
+    auto *tiles = C.rad > kWideRadius ? k_rd_tiles<true> : k_rd_tiles<false>;
+    tiles<<<Pv->ntiles, kTB, 0, s>>>(C, Pv->tile_start, Pv->tile_fill, Pv->recs, Pv->rec_cap,
+                                     reinterpret_cast<const float4 *>(P->col), r->buf, Pv->diag, Pv->tile_est);
     GGB_LAUNCHED();
     stage_end(ST_TILES);
 }
