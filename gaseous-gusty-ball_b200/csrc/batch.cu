@@ -93,7 +93,6 @@ struct GGBBatch {
     SolveParams *prm_host = nullptr;      // [n] pinned
     SolveParams *prm_dev = nullptr;       // [n]
     std::vector<std::vector<int>> groups;  // planets of each launch
-    std::vector<size_t> group_smem;        // dynamic shared memory of each launch
     std::vector<int> blocks;               // blocks of each planet's solve
     int4 *bmap_host = nullptr, *bmap_dev = nullptr;  // [sum of blocks] block -> (planet, block, blocks)
     int bmap_cap = 0;
@@ -164,17 +163,13 @@ static void allocate(GGBBatch *b, const std::vector<int> &grp, int cap) {
 // shares and the block map.
 static void plan(GGBBatch *b) {
     b->groups.clear();
-    b->group_smem.clear();
     b->blocks.assign(b->n, 1);
     std::vector<int> order[2];
     for (int i = 0; i < b->n; i++) order[fluid_solve_mixed(b->F[i])].push_back(i);
     int total = 0;
     for (int m = 0; m < 2; m++) {
         if (order[m].empty()) continue;
-        // the launch's shared memory: the largest of its planets' needs
-        size_t smem = 0;
-        for (int i : order[m]) smem = std::max(smem, pcg_launch_smem(b->prm_host[i]));
-        const int cap = pcg_batch_capacity(smem, m == 1);
+        const int cap = pcg_batch_capacity(m == 1);
         if (b->fixed_blocks >= cap) {
             // every planet alone on the whole launch: one launch per planet,
             // the same blocks (and so the same arithmetic) as fluid_step's solve
@@ -182,7 +177,6 @@ static void plan(GGBBatch *b) {
                 b->blocks[i] = cap;
                 total += cap;
                 b->groups.push_back(std::vector<int>{i});
-                b->group_smem.push_back(smem);
             }
             continue;
         }
@@ -198,7 +192,6 @@ static void plan(GGBBatch *b) {
             }
             for (int i : grp) total += b->blocks[i];
             b->groups.push_back(grp);
-            b->group_smem.push_back(smem);
         }
     }
     if (total > b->bmap_cap) {
@@ -334,8 +327,7 @@ GGB_EXPORT int ggb_batch_step(GGBBatch *b, int steps) {
             const std::vector<int> &grp = b->groups[g];
             int nb = 0;
             for (int i : grp) nb += b->blocks[i];
-            pcg_launch_batch(b->prm_dev, b->bmap_dev + q, nb, fluid_solve_mixed(b->F[grp[0]]) != 0, b->group_smem[g],
-                             base);
+            pcg_launch_batch(b->prm_dev, b->bmap_dev + q, nb, fluid_solve_mixed(b->F[grp[0]]) != 0, base);
             q += nb;
         }
         for (int i = 0; i < b->n; i++) fluid_result_queue(b->F[i]);

@@ -7,20 +7,19 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "ggb_internal.h"
 #include "ggb_solver.h"
 
 namespace ggb {
 
-int pcg_grid_size();
 int pcg_max_blocks();
 int pcg_max_grid_n();
-int pcg_block_size();
 void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks = 0);
-int pcg_check_structured(const LevelDev &F, const LevelDev &C);
-float *pcg_build_rw16(const LevelDev &F, const LevelDev &C);
-double *pcg_dense_map(const SolveParams &prm, int l0);
+void levels_build(const SolveParams &P, LevelSet *out, std::vector<void *> &mem);
+void levels_build_mixed(const SolveParams &P, const LevelSet &plain, LevelSet *out, std::vector<void *> &mem);
+float *pcg_dense_map(const SolveParams &prm, int l0, int ld);
 
 constexpr int kB = 256;
 
@@ -372,12 +371,6 @@ __global__ void k_rsort(int nc, const int *rstart, int *rkey, const float *pw, i
     }
 }
 
-// FP16 copy of a level's slot weights (mixed-precision V-cycle).
-__global__ void k_to_half(size_t n, const float *src, __half *dst) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = __float2half_rn(src[i]);
-}
-
 // ------------------------------------------------------------ private state
 
 struct FluidPriv {
@@ -387,25 +380,21 @@ struct FluidPriv {
     int nlev = 0;
     int *ptap[kMaxLev] = {}, *rstart[kMaxLev] = {}, *ridx[kMaxLev] = {};
     float *pw[kMaxLev] = {}, *rw[kMaxLev] = {};
-    float *lx[kMaxLev] = {}, *lxo[kMaxLev] = {}, *lb[kMaxLev] = {}, *lr[kMaxLev] = {};
     float *r2 = nullptr, *p2 = nullptr;
     double *part = nullptr;
-    double *wpart = nullptr;
     GridBarrier *bar = nullptr;
     SolveResult *res = nullptr;
     SolveResult *res_host = nullptr;
     unsigned int *vmax_bits = nullptr;
     unsigned int *vmax_host = nullptr;
-    int structured[kMaxLev] = {};  // level l -> l+1 transfers follow the index pattern
-    float *rw16[kMaxLev] = {};     // coarse-major structured restriction weights
-    double *dense = nullptr;       // dense map of the V-cycle below the grid levels
-    int nd = 0;
+    LevelSet set[2] = {};           // what vcycle.cu builds for the plain and the mixed solve
+    std::vector<void *> level_mem;  // its device arrays
+    float *sw0 = nullptr, *sw1 = nullptr;  // sweeps of a coarsest level without a dense map
+    float *dense = nullptr;        // dense map of the V-cycle below the grid levels
+    int nd = 0, ld = 0;
     int last_flags = 0;            // kSolve* bits of the last solve
-    // mixed-precision solve (ggb_fluid_set_precision): FP16 level vectors,
-    // FP16 slot weights of the coarse levels, the previous z
+    // mixed-precision solve (ggb_fluid_set_precision): the previous z
     int mixed = 0;
-    __half *hx[kMaxLev] = {}, *hxo[kMaxLev] = {}, *hb[kMaxLev] = {}, *hr[kMaxLev] = {};
-    __half *wh[kMaxLev] = {};
     float *z2 = nullptr;
 };
 
@@ -416,15 +405,14 @@ static FluidPriv *priv_of(const Fluid *F) {
 
 static StencilDev stencil_of(const GridTables *t) {
     StencilDev s;
-    s.wslot_h = nullptr;
     s.N = t->N;
     s.n = t->n;
     s.nring = t->nring;
-    s.lgN = -1;
-    for (int l = 0; l < 31; l++)
-        if ((1 << l) == t->N) s.lgN = l;
+    s.rN = ((1ull << 40) + t->N - 1) / t->N;
     s.wslot = t->wslot;
-    s.wslot_d = t->wslot_d;
+    s.wpad = t->wpad;
+    s.pad = t->N + 1;
+    s.wplane = t->wplane();
     s.ring_nb = t->ring_nb;
     s.ring_w = t->ring_w;
     return s;
@@ -463,13 +451,6 @@ static void build_levels(Fluid *F, FluidPriv *Pv) {
         dev_free(cursor);
         dev_free(rkey);
     }
-    for (int l = 0; l < nlev; l++) {
-        int n = l == 0 ? Pv->grid0->n : Pv->coarse[l].n;
-        Pv->lx[l] = (float *)dev_alloc(sizeof(float) * n);
-        Pv->lxo[l] = (float *)dev_alloc(sizeof(float) * n);
-        Pv->lb[l] = (float *)dev_alloc(sizeof(float) * n);
-        Pv->lr[l] = (float *)dev_alloc(sizeof(float) * n);
-    }
     F->nlev = nlev;
     for (int l = 0; l < nlev; l++) {
         MGLevel *M = &Pv->lev[l];
@@ -482,8 +463,7 @@ static void build_levels(Fluid *F, FluidPriv *Pv) {
     }
 }
 
-constexpr int kBlockLevelMax = 1536;  // levels up to N=16 form the dense coarse map
-
+constexpr int kBlockLevelMax = 1536;  // levels up to N=16 form the dense coarse map (a single level: one block sweeps it)
 static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int maxit) {
     if (F->cs->N > pcg_max_grid_n())
         fail_msg("grids with N > %d exceed the solve kernel's staged window (N = %d)", pcg_max_grid_n(), F->cs->N);
@@ -501,26 +481,12 @@ static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int ma
         LevelDev &L = P.L[l];
         L.S = stencil_of(t);
         L.dinv = t->dinv;
-        if (Pv->mixed) {
-            L.S.wslot_h = Pv->wh[l];
-            L.x = Pv->hx[l];
-            L.xo = Pv->hxo[l];
-            L.b = Pv->hb[l];
-            L.r = Pv->hr[l];
-        } else {
-            L.x = Pv->lx[l];
-            L.xo = Pv->lxo[l];
-            L.b = Pv->lb[l];
-            L.r = Pv->lr[l];
-        }
         if (l + 1 < Pv->nlev) {
             L.ptap = Pv->ptap[l];
             L.pw = Pv->pw[l];
             L.rstart = Pv->rstart[l];
             L.ridx = Pv->ridx[l];
             L.rw = Pv->rw[l];
-            L.structured = Pv->structured[l];
-            L.rw16 = Pv->rw16[l];
         }
     }
     if (mg && Pv->nlev >= 2) {
@@ -547,30 +513,39 @@ static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int ma
     P.part = Pv->part;
     P.bar = Pv->bar;
     P.res = Pv->res;
+    const LevelSet &set = Pv->set[Pv->mixed];
+    for (int l = 0; l <= P.nlev_grid; l++) {
+        LevelDev &L = P.L[l];
+        L.rw16 = set.rw16[l];
+        L.rst = set.rst[l];
+        L.ring_link = set.ring_link[l];
+        L.ring_cell = set.ring_cell[l];
+        if (set.wpad[l]) L.S.wpad = set.wpad[l];
+        L.b = set.b[l];
+        L.xo = set.xo[l];
+        L.r = set.r[l];
+    }
+    P.sw0 = Pv->sw0;
+    P.sw1 = Pv->sw1;
     if (mg && Pv->dense) {
         P.dense = Pv->dense;
         P.nd = Pv->nd;
+        P.ld = Pv->ld;
     }
     return P;
 }
 
-// Structured-transfer flags and the dense coarse map (after build_levels).
+// The dense coarse map, or the buffers of the coarsest level's sweeps (after build_levels).
 static void finish_levels(Fluid *F, FluidPriv *Pv) {
     SolveParams P = solve_params(F, Pv, 0, 1);
-    P.mixed = 0;
-    for (int l = 0; l + 1 < Pv->nlev; l++) {
-        LevelDev Fl = P.L[l], C = P.L[l + 1];
-        Fl.structured = 0;
-        Pv->structured[l] = pcg_check_structured(Fl, C);
-        if (Pv->structured[l]) Pv->rw16[l] = pcg_build_rw16(Fl, C);
-    }
-    if (Pv->nlev >= 2) {
-        P = solve_params(F, Pv, 0, 1);  // with the structured flags
-        int G = P.nlev_grid;
-        if (G < Pv->nlev && P.L[G].S.n <= kBlockLevelMax) {
-            Pv->dense = pcg_dense_map(P, G);
-            Pv->nd = P.L[G].S.n;
-        }
+    if (Pv->nlev >= 2 && P.L[P.nlev_grid].S.n <= kBlockLevelMax) {
+        Pv->nd = P.L[P.nlev_grid].S.n;
+        Pv->ld = (Pv->nd + 3) & ~3;
+        Pv->dense = pcg_dense_map(P, P.nlev_grid, Pv->ld);
+    } else {
+        const size_t n = P.L[Pv->nlev - 1].S.n;
+        Pv->sw0 = (float *)dev_alloc(sizeof(float) * n);
+        Pv->sw1 = (float *)dev_alloc(sizeof(float) * n);
     }
 }
 
@@ -685,14 +660,10 @@ GGB_EXPORT int fluid_init(Fluid *F, const CubeSphere *cs, const FluidParams *prm
         finish_levels(F, Pv);
     } else {
         Pv->nlev = 0;
-        Pv->lx[0] = (float *)dev_alloc(sizeof(float) * n);
-        Pv->lxo[0] = (float *)dev_alloc(sizeof(float) * n);
-        Pv->lb[0] = (float *)dev_alloc(sizeof(float) * n);
-        Pv->lr[0] = (float *)dev_alloc(sizeof(float) * n);
         F->nlev = 0;
     }
-    Pv->part = (double *)dev_alloc(sizeof(double) * 8 * pcg_max_blocks());
-    Pv->wpart = (double *)dev_alloc(sizeof(double) * 1024);
+    levels_build(solve_params(F, Pv, 0, 1), &Pv->set[0], Pv->level_mem);
+    Pv->part = (double *)dev_alloc(sizeof(double) * 4 * pcg_max_blocks());
     Pv->bar = (GridBarrier *)dev_alloc(sizeof(GridBarrier));
     Pv->res = (SolveResult *)dev_alloc(sizeof(SolveResult));
     Pv->vmax_bits = (unsigned int *)dev_alloc(sizeof(unsigned int));
@@ -719,22 +690,14 @@ GGB_EXPORT void fluid_free(Fluid *F) {
         dev_free(Pv->rstart[l]);
         dev_free(Pv->ridx[l]);
         dev_free(Pv->rw[l]);
-        dev_free(Pv->rw16[l]);
-        dev_free(Pv->lx[l]);
-        dev_free(Pv->lxo[l]);
-        dev_free(Pv->lb[l]);
-        dev_free(Pv->lr[l]);
-        dev_free(Pv->hx[l]);
-        dev_free(Pv->hxo[l]);
-        dev_free(Pv->hb[l]);
-        dev_free(Pv->hr[l]);
-        dev_free(Pv->wh[l]);
     }
+    for (void *p : Pv->level_mem) dev_free(p);
+    dev_free(Pv->sw0);
+    dev_free(Pv->sw1);
     dev_free(Pv->z2);
     dev_free(Pv->r2);
     dev_free(Pv->p2);
     dev_free(Pv->part);
-    dev_free(Pv->wpart);
     dev_free(Pv->bar);
     dev_free(Pv->res);
     dev_free(Pv->vmax_bits);
@@ -750,8 +713,7 @@ GGB_EXPORT int ggb_solve_flags(const Fluid *F) { return priv_of(F)->last_flags; 
 
 // Switches the Poisson solve of F between the plain form (mixed = 0: FP32
 // vectors, FP64 stencil accumulation, the upstream CG) and the mixed-precision
-// form (mixed = 1: FP16 V-cycle vectors and coarse slot weights, FP32
-// accumulation, flexible CG).  The buffers of the mixed form are allocated on
+// form (mixed = 1: FP16 V-cycle vectors, FP32 accumulation, flexible CG).  The buffers of the mixed form are allocated on
 // the first switch.  Returns 0, or -1 for a fluid without multigrid.
 GGB_EXPORT int ggb_fluid_set_precision(Fluid *F, int mixed) {
     FluidPriv *Pv = priv_of(F);
@@ -764,20 +726,7 @@ GGB_EXPORT int ggb_fluid_set_precision(Fluid *F, int mixed) {
         return -1;
     }
     if (!Pv->z2) {
-        cudaStream_t s = stream();
-        for (int l = 0; l < Pv->nlev; l++) {
-            const GridTables *t = l == 0 ? Pv->grid0 : &Pv->coarse[l];
-            const size_t n = t->n;
-            Pv->hx[l] = (__half *)dev_alloc(sizeof(__half) * n);
-            Pv->hxo[l] = (__half *)dev_alloc(sizeof(__half) * n);
-            Pv->hb[l] = (__half *)dev_alloc(sizeof(__half) * n);
-            Pv->hr[l] = (__half *)dev_alloc(sizeof(__half) * n);
-            if (l >= 1) {
-                Pv->wh[l] = (__half *)dev_alloc(sizeof(__half) * 4 * n);
-                k_to_half<<<blocks_for((int)std::min<size_t>(4 * n, 1u << 30)), kB, 0, s>>>(4 * n, t->wslot, Pv->wh[l]);
-                GGB_LAUNCHED();
-            }
-        }
+        levels_build_mixed(solve_params(F, Pv, 0, 1), Pv->set[0], &Pv->set[1], Pv->level_mem);
         Pv->z2 = (float *)dev_alloc(sizeof(float) * F->cs->ncells);
         sync();
     }

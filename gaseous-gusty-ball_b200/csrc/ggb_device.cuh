@@ -250,34 +250,30 @@ __device__ __forceinline__ unsigned int atom_add_acq_rel_u32(unsigned int *p, un
 // The arrival is the first global access of a barrier (no generation or error
 // read before it); the error flag and the timeout are checked every 64 polls.
 // nb: the number of blocks that meet at this barrier (the whole grid, or the
-// blocks of one solve inside a batched launch).
+// blocks of one solve inside a batched launch).  One thread's part:
+__device__ __forceinline__ int grid_arrive_wait(GridBarrier *bar, unsigned int nb, unsigned long long limit_ns) {
+    const unsigned int old = atom_add_acq_rel_u32(&bar->count, 1u);
+    const unsigned int target = (old / nb + 1u) * nb;
+    unsigned long long t0 = 0;
+    unsigned int polls = 0;
+    while ((int)(ld_acquire_u32(&bar->count) - target) < 0) {
+        if ((++polls & 63u) == 0) {
+            if (ld_volatile_i32(&bar->err) != 0) return 0;
+            const unsigned long long t = globaltimer_ns();
+            if (polls == 64u) {
+                t0 = t;
+            } else if (t - t0 > limit_ns) {
+                atomicExch(&bar->err, 1);
+                return 0;
+            }
+        }
+    }
+    return 1;
+}
 __device__ __forceinline__ bool grid_sync_nb(GridBarrier *bar, unsigned int nb, unsigned long long limit_ns) {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned int old = atom_add_acq_rel_u32(&bar->count, 1u);
-        const unsigned int target = (old / nb + 1u) * nb;
-        int ok = 1;
-        unsigned long long t0 = 0;
-        unsigned int polls = 0;
-        while ((int)(ld_acquire_u32(&bar->count) - target) < 0) {
-            if ((++polls & 63u) == 0) {
-                if (ld_volatile_i32(&bar->err) != 0) {
-                    ok = 0;
-                    break;
-                }
-                const unsigned long long t = globaltimer_ns();
-                if (polls == 64u) {
-                    t0 = t;
-                } else if (t - t0 > limit_ns) {
-                    atomicExch(&bar->err, 1);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        s_ok = ok;
-    }
+    if (threadIdx.x == 0) s_ok = grid_arrive_wait(bar, nb, limit_ns);
     __syncthreads();
     return s_ok != 0;
 }

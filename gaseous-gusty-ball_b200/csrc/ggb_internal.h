@@ -103,10 +103,8 @@ void fluid_step_solve_params(Fluid *F, GridBarrier *bar, SolveParams *out);
 int fluid_solve_mixed(const Fluid *F);
 double fluid_last_solve_seconds(const Fluid *F);
 void fluid_result_velocity_queue(Fluid *F);
-size_t pcg_launch_smem(const SolveParams &p);
-int pcg_batch_capacity(size_t smem, bool mixed);
-void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, bool mixed, size_t smem,
-                      cudaStream_t s);
+int pcg_batch_capacity(bool mixed);
+void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, bool mixed, cudaStream_t s);
 void render_deposit_queue(Render *r, const Particles *P);
 void render_deposit_collect(Render *r, const Particles *P);
 void particles_advect_queue(Particles *P, const CubeSphere *cs, const float *vel, const double *dt_dev);
@@ -146,7 +144,8 @@ struct GridTables {
     // device-only
     int *ghost = nullptr;
     float *wslot = nullptr;
-    double *wslot_d = nullptr;  // the same four slot weights in FP64 (staged solver phases)
+    float *wpad = nullptr;  // the slot planes with N + 1 zeros before and at least as many after each
+    int wplane() const { return (n + 2 * (N + 1) + 4 + 3) & ~3; }  // their stride
     int *ring_nb = nullptr;
     float *ring_w = nullptr;
     float *dinv = nullptr;

@@ -7,14 +7,22 @@ namespace ggb {
 
 constexpr int kMaxLev = 12;
 
-// One multigrid level on the device.  The level vectors are float in the
-// plain solve and __half in the mixed-precision solve (SolveParams::mixed).
+// Sparse rows of (index, weight bits) taps: step s of row r is tap[s * rows + r].
+// glen: the steps that each 32 rows need (stored steps past a row's own taps
+// have weight 0).
+struct SparseOp {
+    int rows, steps;
+    const int2 *tap;
+    const unsigned char *glen;
+};
+
+// One multigrid level on the device.  The level vectors are float in the plain
+// solve and __half in the mixed-precision solve (SolveParams::mixed).
 struct LevelDev {
     StencilDev S;
     const float *dinv;  // [n] 1 / sum of link weights
-    void *x;            // [n] iterate (pre-smoothed, then corrected)
-    void *xo;           // [n] V-cycle output of this level
-    void *b;            // [n] right-hand side (restricted residual)
+    void *b;            // [n] right-hand side (restricted residual; levels >= 1)
+    void *xo;           // [n] V-cycle output of this level (levels >= 1)
     void *r;            // [n] residual after the pre-smooth
     // transfer to the next coarser level
     const int *ptap;    // [4n] coarse taps of each cell of this level
@@ -22,8 +30,21 @@ struct LevelDev {
     const int *rstart;  // [n_coarse+1] rows of R = P^T
     const int *ridx;    // fine cells of each row (ascending)
     const float *rw;    // weights of each row
-    int structured;     // 1: interior rows of R / P follow the 4x4 / 2x2 index pattern (verified at setup)
-    const float *rw16;  // [16][n_coarse] weights of the structured R rows (coarse-major), or nullptr
+    const float *rw16;  // [16][n_coarse] weights of the interior rows of R (coarse-major), or nullptr when
+                        // the transfers do not follow the 4x4 / 2x2 index pattern
+    SparseOp rst;       // the rows of R of the coarse ring cells (rw16) or of all coarse cells
+    const int2 *ring_link;  // [6 nring][8] the ring cells' links (vcycle.cu)
+    const int *ring_cell;   // [6 nring] ring cell | its on-face lanes << 24
+};
+
+// What levels_build (vcycle.cu) makes of a hierarchy, per precision.
+struct LevelSet {
+    const float *rw16[kMaxLev];
+    SparseOp rst[kMaxLev];
+    const int2 *ring_link[kMaxLev];
+    const int *ring_cell[kMaxLev];
+    const float *wpad[kMaxLev];  // nullptr: the grid's own
+    void *b[kMaxLev], *xo[kMaxLev], *r[kMaxLev];
 };
 
 // Status bits of a solve (SolveResult::flags; also ggb_solve_flags).
@@ -44,11 +65,11 @@ struct SolveResult {
 };
 
 struct SolveParams {
-    int mixed;           // 1: V-cycle vectors (and coarse slot weights) in FP16 with FP32 accumulation,
-                         //    flexible (Polak-Ribiere) CG; 0: FP32 vectors, FP64 accumulation
+    int mixed;           // 1: V-cycle vectors in FP16 with FP32 accumulation, flexible (Polak-Ribiere) CG;
+                         //    0: FP32 vectors, FP64 accumulation
     int nlev;            // >= 1 when multigrid, 0 for the Jacobi preconditioner
     int nlev_grid;       // non-coarsest levels 0..nlev_grid-1 run grid-wide
-    int coarse_on_grid;  // coarsest level swept grid-wide (else by block 0)
+    int coarse_on_grid;  // coarsest level swept grid-wide (else the dense map)
     int coarse_sweeps;   // Jacobi sweeps on the coarsest level (upstream: 60)
     int remove_mean;     // project the mean out of omega first
     int maxit;
@@ -59,14 +80,15 @@ struct SolveParams {
     float *omega, *psi;
     float *r, *r2, *p, *p2, *Ap, *z;  // level-0 CG vectors (r / p ping-pong)
     float *z2;           // mixed: the previous z (z / z2 ping-pong for the flexible beta)
-    double *part;        // [RED_N][gridDim.x] per-block partial sums
     unsigned long long *trace;  // optional: block 0 stamps %globaltimer at phase marks
     int trace_cap;
+    double *part;        // [2][2][blocks] the blocks' sums at the last two barriers
     GridBarrier *bar;
     SolveResult *res;
     // dense form of the V-cycle below the grid levels: xo_G = D b_G
-    const double *dense;  // [nd][nd] row-major, or nullptr
-    int nd;               // cells of level nlev_grid
+    float *sw0, *sw1;    // the coarsest level's sweeps (coarse_on_grid)
+    const float *dense;  // [nd][ld] row-major (rows padded with zeros to ld), or nullptr
+    int nd, ld;          // cells of level nlev_grid; row stride, a multiple of 4
 };
 
 }  // namespace ggb

@@ -12,10 +12,10 @@ namespace ggb {
 
 struct StencilDev {
     int N, n, nring;
-    int lgN;              // log2(N) when N is a power of two, else -1
+    unsigned long long rN;  // ceil(2^40 / N)
     const float *wslot;   // [4][n]: E, N, NE, NW weights (0 = no link)
-    const double *wslot_d;  // the same in FP64
-    const __half *wslot_h;  // the same in FP16 (mixed-precision V-cycle, levels >= 1), or nullptr
+    const float *wpad;    // the four planes with at least pad zeros before and after each, plane stride wplane (x 4)
+    int pad, wplane;
     const int *ring_nb;   // [6*nring][8], -1 terminated
     const float *ring_w;  // [6*nring][8]
 };
@@ -35,18 +35,14 @@ __device__ __forceinline__ void cell_fij(int c, int N, int &f, int &i, int &j) {
     i = rem - j * N;
 }
 
-// cell_fij for a level's stencil: shifts and masks when N is a power of two
-// (an integer division takes some twenty instructions), the division otherwise.
+// cell_fij for a level's stencil: the divisions as multiplications by rN =
+// ceil(2^40 / N) (exact: c < 6 N^2 <= 2^24 and N <= 1535, so c N < 2^40), which take a
+// fraction of an integer division's instructions.
 __device__ __forceinline__ void cell_fij(const StencilDev &S, int c, int &f, int &i, int &j) {
-    const int l = S.lgN;
-    if (l >= 0) {
-        f = c >> (2 * l);
-        const int rem = c & ((1 << (2 * l)) - 1);
-        j = rem >> l;
-        i = rem & ((1 << l) - 1);
-    } else {
-        cell_fij(c, S.N, f, i, j);
-    }
+    const int row = (int)(((unsigned long long)(unsigned)c * S.rN) >> 40);  // c / N
+    f = (int)(((unsigned long long)(unsigned)row * S.rN) >> 40);
+    i = c - row * S.N;
+    j = row - f * S.N;
 }
 
 // The links of a boundary-ring cell that leave the face: all eight (neighbour,
@@ -134,32 +130,6 @@ __device__ __forceinline__ void ring_cell_of_rank(int R, int N, int nring, int &
         j = N - 1;
         i = q - (3 * N - 4);
     }
-}
-
-// K at cell c with the window's values x[k] and FP64 slot weights w0..w3[k]
-// all staged in shared memory (indexed by cell; the window spans [c - N - 1,
-// c + N + 1] for every cell c of the block's range, zero-filled where it
-// runs past the ends of the grid).  One branch-free formula serves every
-// cell: a slot whose link would leave the face has weight 0 in the layout
-// (also where the neighbouring index wraps to another row or face), so its
-// term adds an exact zero.  A boundary-ring cell adds the staged sum of its
-// links that leave the face, rsum[ring rank - r0].
-template <class A>
-__device__ __forceinline__ A apply_k_smem(const StencilDev &S, int c, A xc, const A *x, const A *wE, const A *wN,
-                                          const A *wNE, const A *wNW, const A *rsum, int r0) {
-    const int N = S.N;
-    int f, i, j;
-    cell_fij(S, c, f, i, j);
-    A s = wE[c] * (xc - x[c + 1]);
-    s += wN[c] * (xc - x[c + N]);
-    s += wNE[c] * (xc - x[c + N + 1]);
-    s += wNW[c] * (xc - x[c + N - 1]);
-    s += wE[c - 1] * (xc - x[c - 1]);
-    s += wN[c - N] * (xc - x[c - N]);
-    s += wNE[c - N - 1] * (xc - x[c - N - 1]);
-    s += wNW[c - N + 1] * (xc - x[c - N + 1]);
-    if (i == 0 || j == 0 || i == N - 1 || j == N - 1) s += rsum[f * S.nring + ring_rank_in_face(i, j, N) - r0];
-    return s;
 }
 
 // The links of cell c as up to 8 (neighbour, weight) pairs; unused pairs have

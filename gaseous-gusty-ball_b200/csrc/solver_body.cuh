@@ -1,27 +1,36 @@
-// solver_body.cuh — the device code of the persistent solve kernel k_pcg
-// (constants, staged stencil phases, V-cycle, PCG body), included inside a
-// namespace by solver.cu (the 512-thread kernel and everything else) and by
-// solver_wide.cu (the 640-thread kernel).  Two translation units keep the
-// compiler's inlining and register allocation of each kernel independent of
-// the other: with both block sizes in one unit the 512-thread plain kernel
-// lost its inlined V-cycle and ran 20 % slower.
+// solver_body.cuh — the device code of the persistent solve kernels k_pcg /
+// k_pcg_batch (constants, stencil phases, V-cycle, PCG body), included by
+// solver.cu inside its namespace.
 //
 // Upstream: src/fluid.c:41-160 (multigrid), :264-275 (mean), :290-358 (PCG).
-// Must be included after ggb_internal.h and ggb_solver.h, inside a namespace.
+//
+// A solve is a chain of some 130 phases of 3 to 10 us, each executed once per
+// grid barrier; what bounds it is the latency of a phase (barrier, one round of
+// loads, the instructions of one warp), not bytes.  So each kind of phase is
+// inlined once, in loops over levels and iterations (a variant with 640 KB of code
+// spent a seventh of its stall cycles on instruction fetch), no static operand is
+// read between a barrier and the values that wait for it, and the window of a
+// phase holds FP32 values only.  Solve in ms, before (values, four FP64 weights
+// and three inputs of every window cell staged anew in each phase) and after:
+// N = 64 0.273, 0.242; N = 256 0.869, 0.757; N = 512 2.33, 1.92; mixed 0.852,
+// 0.775 and 2.23, 1.93.  The FP32 and FP16 roundings of every vector are unchanged.
 
-constexpr int kPB = 512;            // threads per block of the persistent kernel
-constexpr int kPBWide = 640;        // ... for grids from kWideMinN on (more loads in flight per SM)
-constexpr int kWideMinN = 384;      // measured: 512 threads faster at N = 256, 640 at N = 512
-constexpr int kRedBlock = 1024;     // block size the reductions are written for (absent warps add zeros)
-constexpr double kOmegaJ = 0.8;     // upstream MG_OMEGA
+constexpr int kBlockSweepMax = 1536;  // cells of a level that one block sweeps in shared memory
+constexpr int kPB = 512;          // threads per block of the persistent kernel
+constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh the phases' latency
+constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 256 0.756 / 0.906, 448 1.57 / 1.68, 512 1.97 / 1.92
+constexpr int kChunk = 3072;      // cells of a stencil chunk
+constexpr double kOmegaJ = 0.8;      // upstream MG_OMEGA
 constexpr double kCorrScale = 1.0;  // upstream MG_CORR_SCALE
-constexpr int kStageCap = 3584;     // cells of a block's staged window (value + 4 slot weights FP64, 3 FP32 own inputs)
-constexpr int kRingCap = 1024;      // boundary-ring cells of one staged sub-range (their off-face link sums)
-constexpr int kStageWords = kStageCap * 5 + (kStageCap * 3 + 1) / 2 + kRingCap;  // in doubles
-constexpr size_t kStageBytes = (size_t)kStageWords * sizeof(double);
-static_assert((kStageCap * 3) % 2 == 0, "the ring sums follow the own-input arrays on an 8-byte boundary");
-
-enum { RED_BB = 0, RED_RR, RED_PAP, RED_RZ, RED_MEAN, RED_AREA, RED_RZO, RED_N };
+// Shared memory of a block: the value window of a chunk (FP32) and the slot
+// weights of every grid level's window (each level of N <= 512 in its own
+// region).
+constexpr int kMaxN = 1535;
+constexpr int kWinCap = (kChunk + 2 * kMaxN + 2 + 3) & ~3;  // whole 16-byte groups: the pool follows
+static_assert(kWinCap >= 3 * kBlockSweepMax, "x, xo and b of a level that one block sweeps");
+constexpr int kSlotPool = 34816;
+static_assert(kSlotPool >= 4 * (kChunk + 2 * kMaxN + 2 + 8), "a chunk's slot weights fit");
+constexpr size_t kStageBytes = (kWinCap + (size_t)kSlotPool) * sizeof(float);
 
 // Storage (V) and accumulation (A) types of the two precisions.
 template <bool MP>
@@ -37,18 +46,16 @@ struct Prec<true> {
 
 __device__ __forceinline__ float ldv(const float *p, int k) { return p[k]; }
 __device__ __forceinline__ float ldv(const __half *p, int k) { return __half2float(p[k]); }
+// four values, 4-element aligned
+__device__ __forceinline__ float4 ldv4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 ldv4(const __half *p) {
+    const uint2 u = *reinterpret_cast<const uint2 *>(p);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 __device__ __forceinline__ void stv(float *p, int k, float v) { p[k] = v; }
 __device__ __forceinline__ void stv(__half *p, int k, float v) { p[k] = __float2half_rn(v); }
-// store and return the stored value
-__device__ __forceinline__ float stv_get(float *p, int k, float v) {
-    p[k] = v;
-    return v;
-}
-__device__ __forceinline__ float stv_get(__half *p, int k, float v) {
-    const __half h = __float2half_rn(v);
-    p[k] = h;
-    return __half2float(h);
-}
 // v as the storage type would hold it (rounded to FP16 in the mixed solve)
 template <bool MP>
 __device__ __forceinline__ float as_stored(float v) {
@@ -59,79 +66,126 @@ __device__ __forceinline__ typename Prec<MP>::V *lv(void *p) {
     return static_cast<typename Prec<MP>::V *>(p);
 }
 
-// Scale factors of the mixed V-cycle's transfers (1 in the plain solve).
-template <bool MP>
-__device__ __forceinline__ float restrict_scale() {
-    return MP ? 0.25f : 1.0f;
-}
-template <bool MP>
-__device__ __forceinline__ float prolong_scale() {
-    return MP ? 4.0f : 1.0f;
-}
-
-// Slot weight at index q (= s * n + cell) of a level's FP64 (plain), FP16
-// (mixed, when present) or FP32 slot table, as the stencil's accumulation type.
-template <bool MP>
-__device__ __forceinline__ typename Prec<MP>::A slot_w(const double *wd, const float *wf, const __half *wh, int q) {
-    if (MP) {
-        if (wh) return __half2float(wh[q]);
-        return __ldg(wf + q);
-    }
-    return __ldg(wd + q);
-}
-
-// The block's place in its solve's grid (its "virtual grid"): the whole
-// launch for a single solve (blockIdx.x of gridDim.x), or the share of the
-// blocks of a batched launch that one planet's solve runs on.
+// This block's solve: its parameters, its place in the solve's grid (its
+// "virtual grid": the whole launch, or the share of the blocks of a batched
+// launch that one planet's solve runs on), and its ranges of the levels.
+__shared__ SolveParams sP;
 __shared__ int s_vgrid[2];
+__shared__ int s_range[kMaxLev][2];
+// Where a level's slot weights lie in the pool: offset, plane stride, and 1
+// when the block's range is one chunk in a region of its own (loaded once per
+// solve).
+__shared__ int s_slot[kMaxLev][3];
+__shared__ double s_warp[2][32];
+__shared__ double s_total[2];  // the sums of the last vsync
+__shared__ double s_late;      // a sum published at the barrier before (vsync)
+__shared__ int s_epoch;        // barriers passed
+__shared__ int s_ok;
 __device__ __forceinline__ int vb() { return s_vgrid[0]; }
 __device__ __forceinline__ int vnb() { return s_vgrid[1]; }
+// The warps of the virtual grid numbered across its blocks (a short list of
+// work items then takes a few warps of every block, next to other work, rather
+// than all warps of a few blocks).
+__device__ __forceinline__ int vwarp() { return (int)(threadIdx.x >> 5) * vnb() + vb(); }
+__device__ __forceinline__ int vwarps() { return (int)(blockDim.x >> 5) * vnb(); }
+extern __shared__ __align__(16) unsigned char s_dyn[];
+__device__ __forceinline__ float *s_win() { return reinterpret_cast<float *>(s_dyn); }
+
+
+__device__ __forceinline__ float *s_pool() { return s_win() + kWinCap; }
 
 // Phase trace (diagnostics): block 0, thread 0 records (mark, %globaltimer).
 __device__ int g_trace_n;
-__device__ __forceinline__ void trace_mark(const SolveParams &P, int mark) {
-    if (P.trace && vb() == 0 && threadIdx.x == 0) {
-        int k = g_trace_n;
-        if (k < P.trace_cap) {
-            P.trace[2 * k] = (unsigned long long)mark;
-            P.trace[2 * k + 1] = globaltimer_ns();
+__device__ __noinline__ void trace_mark(int mark) {
+    if (vb() == 0 && threadIdx.x == 0) {
+        const int k = g_trace_n;
+        if (k < sP.trace_cap) {
+            sP.trace[2 * k] = (unsigned long long)mark;
+            sP.trace[2 * k + 1] = globaltimer_ns();
             g_trace_n = k + 1;
         }
     }
 }
+#define TRACE(mark)                    \
+    do {                               \
+        if (sP.trace) trace_mark(mark); \
+    } while (0)
 
 // GRID_LOOP: over the block's virtual grid (only inside k_pcg / k_pcg_batch,
 // which set it); KERNEL_LOOP: over the launch's real grid (set-up kernels).
 #define GRID_LOOP(c, n) for (int c = vb() * blockDim.x + threadIdx.x; c < (n); c += vnb() * blockDim.x)
 #define KERNEL_LOOP(c, n) for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < (n); c += gridDim.x * blockDim.x)
+// OWN_LOOP: the cells of this block's level-0 range
+#define OWN_LOOP(c) for (int c = s_range[0][0] + (int)threadIdx.x; c < s_range[0][1]; c += blockDim.x)
 #define BLOCK_LOOP(c, n) for (int c = threadIdx.x; c < (n); c += blockDim.x)
-#define SYNC_OR(fail)              \
-    do {                           \
-        if (!vsync(P)) fail;       \
-    } while (0)
 
-struct Red {
-    double v[kRedBlock / 32 + 2];
-};
-
-// Barrier of the blocks of one solve (a block barrier when the solve has one block).
-__device__ __forceinline__ bool vsync(const SolveParams &P) {
-    if (vnb() == 1) {
-        __syncthreads();
-        return true;
+// Barrier of the blocks of one solve, and the sums of nv (0..2) values over all
+// their threads.  A block leaves its sums in its row of the partials (two sets
+// in turn: a set is written again only after every block has passed the barrier
+// behind its reads) and arrives at the counter; after the barrier one warp reads
+// all rows, in an order that depends on indices only, and leaves the totals in
+// s_total in every block.  With late, the totals are not read here but by the
+// next vsync called with fetch, by a second warp while the first one waits, and
+// left in s_late: a sum whose only use is the convergence test costs no round
+// trip that way.  (Arrival and sums in one message, every block polling every
+// other's slot, measured 4 us a barrier against 1.7 + 1.2.)
+__device__ __forceinline__ double rows_total(const double *row, int nb, int lane) {
+    double v = 0;
+#pragma unroll 5
+    for (int k = lane; k < nb; k += 32) v += __ldcg(row + k);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ bool vsync(int nv, double v0, double v1, bool late = false, bool fetch = false) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = vnb(), epoch = s_epoch;
+    if (nv > 0) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+        if (lane == 0) s_warp[0][warp] = v0;
     }
-    return grid_sync_nb(P.bar, (unsigned)vnb(), kBarrierTimeoutNs);
+    if (nv > 1) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+        if (lane == 0) s_warp[1][warp] = v1;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        if (nv > 0) {
+            v0 = lane < (int)blockDim.x / 32 ? s_warp[0][lane] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+        }
+        if (nv > 1) {
+            v1 = lane < (int)blockDim.x / 32 ? s_warp[1][lane] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+        }
+        double *row = sP.part + (epoch & 1) * 2 * nb;
+        int ok = 1;
+        if (lane == 0) {
+            if (nv > 0) row[vb()] = v0;
+            if (nv > 1) row[nb + vb()] = v1;
+            if (nb > 1) ok = grid_arrive_wait(sP.bar, (unsigned)nb, kBarrierTimeoutNs);
+        }
+        __syncwarp();
+        if (nv > 0 && !late) {
+            v0 = rows_total(row, nb, lane);
+            if (nv > 1) v1 = rows_total(row + nb, nb, lane);
+        }
+        if (lane == 0) {
+            s_total[0] = v0;
+            s_total[1] = v1;
+            s_ok = ok;
+            s_epoch = epoch + 1;
+        }
+    } else if (warp == 1 && fetch) {
+        const double t = rows_total(sP.part + ((epoch + 1) & 1) * 2 * nb, nb, lane);
+        if (lane == 0) s_late = t;
+    }
+    __syncthreads();
+    return s_ok != 0;
 }
-
-__device__ __forceinline__ void put_partial(const SolveParams &P, int which, double v, double *s_red) {
-    double t = block_sum<kRedBlock>(v, s_red);
-    if (threadIdx.x == 0) P.part[which * vnb() + vb()] = t;
-}
-__device__ __forceinline__ double get_total(const SolveParams &P, int which, double *s_red) {
-    return sum_partials<kRedBlock>(P.part + which * vnb(), vnb(), s_red);
-}
-
-// ---- staged stencil phases ------------------------------------------------
 
 // This block's contiguous range of a level's n = 6 N^2 cells (face-major).
 // With at least 6 blocks every face gets a whole number of blocks (face f:
@@ -155,10 +209,10 @@ __device__ __forceinline__ void block_range(int n, int N, int &c0, int &c1) {
     c1 = (int)(f * nf + nf * (b - b0 + 1) / m);
 }
 
-__device__ unsigned long long *g_stage_trace;  // diagnostics: block 0 stamps staging / compute ends
+__device__ unsigned long long *g_stage_trace;  // diagnostics: block 0 stamps the stencil phases
 __device__ int g_stage_trace_n;
 __device__ int g_stage_trace_all;  // 1: every block records, mark | block << 16
-__device__ __forceinline__ void stage_mark(int mark) {
+__device__ __noinline__ void stage_mark(int mark) {
     unsigned long long *t = g_stage_trace;
     if (!t || threadIdx.x != 0) return;
     if (g_stage_trace_all) {
@@ -177,330 +231,276 @@ __device__ __forceinline__ void stage_mark(int mark) {
     }
 }
 
-// Inputs of a cell of the block's own range: a, b, c are staged in shared
-// memory for the compute loop; d stays in the staging thread (for commit).
-struct Own {
-    float a, b, c, d;
+__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Starts the copy of the slot weights of the window of chunk [s0, s1) of level
+// l: cell k of plane p at pool[offset + p * stride + k - (s0 - N - 1) + shift],
+// shift = the cells by which the copy starts before the window for 16-byte
+// alignment.
+__device__ __forceinline__ int slot_shift(const StencilDev &S, int s0) { return (s0 - S.N - 1 + S.pad) & 3; }
+__device__ __noinline__ void slots_load(int l, int s0, int s1) {
+    const StencilDev &S = sP.L[l].S;
+    const int a = (s0 - S.N - 1 + S.pad) & ~3, groups = (s1 - s0 + 2 * (S.N + 1) + 3 + 3) >> 2;
+    float *dst = s_pool() + s_slot[l][0];
+    const int cap = s_slot[l][1];
+    for (int p = 0; p < 4; p++)
+        for (int k = 4 * threadIdx.x; k < 4 * groups; k += 4 * blockDim.x)
+            if (a + k + 4 <= S.wplane) cp_async16(dst + p * cap + k, S.wpad + (size_t)p * S.wplane + a + k);
+}
+
+// Ranges of every level, slot regions of level 0 and the grid levels, and the
+// slot weights that stay in shared memory for the whole solve (their copies
+// complete at the first stencil phase's wait).
+__device__ __noinline__ void block_setup() {
+    const int levels = max(sP.nlev, 1), slots = max(sP.nlev_grid, 1);
+    if (threadIdx.x == 0) {
+        int at = 0;
+        bool shared = false;
+        for (int l = 0; l < levels; l++) {
+            const StencilDev &S = sP.L[l].S;
+            int c0, c1;
+            block_range(S.n, S.N, c0, c1);
+            s_range[l][0] = c0;
+            s_range[l][1] = c1;
+            if (l >= slots) continue;
+            const int cap = (min(c1 - c0, kChunk) + 2 * (S.N + 1) + 8 + 3) & ~3;
+            const bool own = at + 4 * cap <= kSlotPool;
+            shared |= !own;
+            s_slot[l][0] = own ? at : 0;
+            s_slot[l][1] = cap;
+            s_slot[l][2] = own && c1 - c0 <= kChunk;
+            if (own) at += 4 * cap;
+        }
+        if (shared) s_slot[0][2] = 0;  // another level's weights pass through level 0's region
+    }
+    __syncthreads();
+    for (int l = 0; l < slots; l++)
+        if (s_slot[l][2]) slots_load(l, s_range[l][0], s_range[l][1]);
+}
+
+// K x at interior cell c from the window (x[k], k = cell index) and the slot
+// weights w0..w3 (indexed by cell) in shared memory.
+// (A slot weight is finite and not negative: widening it to FP64 by its bits, with 2^-127 for
+// 0, takes three integer instructions in place of a conversion at a quarter of
+// their rate.)
+__device__ __forceinline__ double widen(float w, double) {
+    const unsigned b = __float_as_uint(w);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+__device__ __forceinline__ float widen(float w, float) { return w; }
+template <class A>
+__device__ __forceinline__ A apply_window(int c, int N, const float *x, const float *w0, const float *w1,
+                                          const float *w2, const float *w3) {
+    const A xc = x[c];
+    A s = widen(w0[c], A()) * (xc - (A)x[c + 1]);
+    s += widen(w1[c], A()) * (xc - (A)x[c + N]);
+    s += widen(w2[c], A()) * (xc - (A)x[c + N + 1]);
+    s += widen(w3[c], A()) * (xc - (A)x[c + N - 1]);
+    s += widen(w0[c - 1], A()) * (xc - (A)x[c - 1]);
+    s += widen(w1[c - N], A()) * (xc - (A)x[c - N]);
+    s += widen(w2[c - N - 1], A()) * (xc - (A)x[c - N - 1]);
+    s += widen(w3[c - N + 1], A()) * (xc - (A)x[c - N + 1]);
+    return s;
+}
+
+__device__ __forceinline__ bool is_ring(const StencilDev &S, int c) {
+    int f, i, j;
+    cell_fij(S, c, f, i, j);
+    return i == 0 || j == 0 || i == S.N - 1 || j == S.N - 1;
+}
+
+// cell(c, x(c), (K x)(c)) for every cell of level l: x(k) = load(k) is FP32; the
+// sums are FP64 in the plain solve and FP32 in the mixed one, there in the order
+// of the links (on the face E, N, NE, NW, W, S, SW, SE, then the sum of those
+// that leave it).  Boundary-ring cells take eight adjacent threads of the
+// virtual grid each, one per link.  The other cells of this block's range go in
+// chunks: the values of the chunk and N + 1 cells on either side to shared
+// memory, each computed once, and the slot weights by cp.async; then eight links
+// per cell from shared memory.  Bound by latency: a barrier, one round of loads
+// and the reduction, since nothing static is read after the barrier when the
+// range is one chunk (up to N = 256), and by the loads' bandwidth beyond.  Ends
+// with a block barrier.
+struct RingPre {  // a thread's first ring link, read before the grid barrier
+    int2 q;
+    int own;      // ring cell | its on-face lanes << 24
+};
+__device__ __forceinline__ void ring_load(const LevelDev &L, int e, RingPre &R) {
+    R.q = __ldg(L.ring_link + e);
+    R.own = __ldg(L.ring_cell + (e >> 3));
+}
+__device__ __forceinline__ void ring_prefetch(int l, RingPre &R) {
+    const LevelDev &L = sP.L[l];
+    ring_load(L, min(32 * vwarp() + (int)(threadIdx.x & 31), 48 * L.S.nring - 1), R);
+}
+template <bool MP, class Load, class Cell>
+__device__ __forceinline__ void stencil_phase(int l, RingPre &R, Load load, Cell cell) {
+    using A = typename Prec<MP>::A;
+    const LevelDev &L = sP.L[l];
+    const StencilDev &S = L.S;
+    const int N = S.N, n = S.n, bs = blockDim.x, tid = threadIdx.x, lane = tid & 31;
+    const int c0 = s_range[l][0], c1 = s_range[l][1];
+    stage_mark(1);
+    const int total = 48 * S.nring, stride = 32 * vwarps();
+#pragma unroll 1
+    for (int e0 = 32 * vwarp(); e0 < total; e0 += stride) {
+        const int c = R.own & 0xffffff;
+        const float xo = load(c), xn = load(R.q.x);
+        const A d = (A)xo - (A)xn, w = (A)__int_as_float(R.q.y);
+        A v;
+        if (MP) {
+            const unsigned on = (unsigned)R.own >> 24;
+            A wk[kMaxNb], dk[kMaxNb], t = 0;
+#pragma unroll
+            for (int k = 0; k < kMaxNb; k++) {
+                const A wl = __shfl_sync(0xffffffffu, w, k, 8);
+                dk[k] = __shfl_sync(0xffffffffu, d, k, 8);
+                wk[k] = on >> k & 1u ? wl : 0;
+                if (!(on >> k & 1u)) t += wl * dk[k];
+            }
+            v = wk[0] * dk[0];  // apply_window's chain
+            v += wk[1] * dk[1];
+            v += wk[2] * dk[2];
+            v += wk[3] * dk[3];
+            v += wk[4] * dk[4];
+            v += wk[5] * dk[5];
+            v += wk[6] * dk[6];
+            v += wk[7] * dk[7];
+            v += t;
+        } else {
+            v = w * d;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        if (e0 + lane < total && (lane & 7) == 0) cell(c, xo, v);
+        if (e0 + stride < total) ring_load(L, min(e0 + stride + lane, total - 1), R);
+    }
+    float *win = s_win();
+#pragma unroll 1
+    for (int s0 = c0; s0 < c1; s0 += kChunk) {
+        const int s1 = min(c1, s0 + kChunk);
+        const int w0 = s0 - N - 1, w1 = s1 + N + 1;  // cells outside [0, n) stage as zeros
+        if (!s_slot[l][2]) slots_load(l, s0, s1);
+#pragma unroll 4
+        for (int k = w0 + tid; k < w1; k += bs) win[k - w0] = k >= 0 && k < n ? load(k) : 0.f;
+        cp_async_wait();
+        __syncthreads();
+        const float *x = win - w0;
+        const int cap = s_slot[l][1];
+        const float *wE = s_pool() + s_slot[l][0] + slot_shift(S, s0) - w0;
+#pragma unroll 1
+        for (int c = s0 + tid; c < s1; c += bs)
+            if (!is_ring(S, c))
+                cell(c, x[c], apply_window<A>(c, N, x, wE, wE + cap, wE + 2 * cap, wE + 3 * cap));
+        __syncthreads();
+    }
+    stage_mark(2);
+}
+
+// ---- sparse rows ------------------------------------------------------------
+
+// The sum of a row's products, each rounded to FP32: in FP64 (plain), or as an
+// FP32 FMA chain in the order of the taps (mixed).
+template <bool MP>
+struct DotAcc {
+    typename Prec<MP>::A a = 0;
+    __device__ __forceinline__ void add(float w, float x) {
+        if (MP)
+            a = __fmaf_rn(w, x, (float)a);
+        else
+            a += (typename Prec<MP>::A)__fmul_rn(w, x);
+    }
 };
 
-// cell(c, x, wE, wN, wNE, wNW, rsum, r0, o) for every cell c of this block's
-// range of a level.  Over the stencil window of the current sub-range, x[k] =
-// load(k, mine, o) and the four slot weights are staged (accumulation type A:
-// FP64 plain, FP32 mixed) in shared memory; for the cells of the sub-range
-// (mine) load also fills o, whose a, b, c are staged too, and commit(k, o)
-// then performs the cell's side effects (global stores) after the loads of
-// the pass are issued.  load must not store.  The links that leave a face
-// (boundary-ring cells) are summed while staging as well: rsum[ring rank - r0]
-// = sum_k w_k (x(c) - x(nb_k)), one thread per ring cell.  All global loads
-// happen while staging, where they are independent, so the compute loop reads
-// shared memory only.  Ends with a block barrier.
-template <bool MP, class Load, class Commit, class Cell>
-__device__ __forceinline__ void staged(const StencilDev &S, double *raw, Load load, Commit commit, Cell cell) {
-    using A = typename Prec<MP>::A;
-    const int N = S.N, n = S.n, nring = S.nring, bs = blockDim.x, tid = threadIdx.x;
-    int c0, c1;
-    block_range(n, N, c0, c1);
-    const int halo = N + 1;
-    const int sub = kStageCap - 2 * halo;
-    A *buf = reinterpret_cast<A *>(raw);
-    A *bx = buf, *b0 = buf + kStageCap, *b1 = buf + 2 * kStageCap, *b2 = buf + 3 * kStageCap, *b3 = buf + 4 * kStageCap;
-    float *oa = reinterpret_cast<float *>(buf + 5 * kStageCap), *ob = oa + kStageCap, *oc = ob + kStageCap;
-    A *rs = reinterpret_cast<A *>(oc + kStageCap);
-    // the slot tables, read once into registers (not per window cell)
-    const double *wd = S.wslot_d;
-    const float *wf = S.wslot;
-    const __half *wh = S.wslot_h;
-    stage_mark(1);
-    for (int s0 = c0; s0 < c1;) {
-        int s1 = min(c1, s0 + sub);
-        const int r0 = ring_rank_below(s0, N, nring);
-        int r1 = ring_rank_below(s1, N, nring);
-        if (r1 - r0 > kRingCap) {  // end the sub-range before its (kRingCap+1)-th ring cell
-            r1 = r0 + kRingCap;
-            int f, i, j;
-            ring_cell_of_rank(r1, N, nring, f, i, j);
-            s1 = (f * N + j) * N + i;
-        }
-        const int w0 = s0 - halo, w1 = s1 + halo;  // cells outside [0, n) stage as zeros
-        // The ring tables are in ring-rank order: this sub-range's boundary-ring
-        // cells are rows r0..r1-1, one thread per ring cell.  The first row of
-        // each thread (its eight links as two 16-byte loads each) and its own
-        // value are fetched before the window loop so that their latency
-        // overlaps it.
-        const int nr = r1 - r0;
-        const int4 *rn4 = reinterpret_cast<const int4 *>(S.ring_nb) + 2 * (size_t)r0;
-        const float4 *rw4 = reinterpret_cast<const float4 *>(S.ring_w) + 2 * (size_t)r0;
-        int4 fo0 = make_int4(-1, -1, -1, -1), fo1 = fo0;
-        float4 fw0 = make_float4(0.f, 0.f, 0.f, 0.f), fw1 = fw0;
-        A fvc = 0;
-        if (tid < nr) {
-            fo0 = __ldg(rn4 + 2 * tid);
-            fo1 = __ldg(rn4 + 2 * tid + 1);
-            fw0 = __ldg(rw4 + 2 * tid);
-            fw1 = __ldg(rw4 + 2 * tid + 1);
-            int f, i, j;
-            ring_cell_of_rank(r0 + tid, N, nring, f, i, j);
-            Own none;
-            fvc = load((f * N + j) * N + i, false, none);
-        }
-        // window: values and slot weights, two cells per thread per pass with
-        // every global load of both issued before any shared-memory store
-        for (int k = w0 + tid; k < w1; k += 2 * bs) {
-            const int k2 = k + bs;
-            const bool two = k2 < w1;
-            const bool in1 = k >= s0 && k < s1, in2 = two && k2 >= s0 && k2 < s1;
-            Own o1{0.f, 0.f, 0.f, 0.f}, o2{0.f, 0.f, 0.f, 0.f};
-            A e1 = 0, n1 = 0, ne1 = 0, nw1 = 0, v1 = 0;
-            if (k >= 0 && k < n) {
-                e1 = slot_w<MP>(wd, wf, wh, k);
-                n1 = slot_w<MP>(wd, wf, wh, n + k);
-                ne1 = slot_w<MP>(wd, wf, wh, 2 * n + k);
-                nw1 = slot_w<MP>(wd, wf, wh, 3 * n + k);
-                v1 = load(k, in1, o1);
-            }
-            A e2 = 0, n2 = 0, ne2 = 0, nw2 = 0, v2 = 0;
-            if (two && k2 >= 0 && k2 < n) {
-                e2 = slot_w<MP>(wd, wf, wh, k2);
-                n2 = slot_w<MP>(wd, wf, wh, n + k2);
-                ne2 = slot_w<MP>(wd, wf, wh, 2 * n + k2);
-                nw2 = slot_w<MP>(wd, wf, wh, 3 * n + k2);
-                v2 = load(k2, in2, o2);
-            }
-            if (in1) commit(k, o1);
-            if (in2) commit(k2, o2);
-            int q = k - w0;
-            bx[q] = v1;
-            b0[q] = e1;
-            b1[q] = n1;
-            b2[q] = ne1;
-            b3[q] = nw1;
-            if (in1) {
-                oa[k - s0] = o1.a;
-                ob[k - s0] = o1.b;
-                oc[k - s0] = o1.c;
-            }
-            if (two) {
-                q = k2 - w0;
-                bx[q] = v2;
-                b0[q] = e2;
-                b1[q] = n2;
-                b2[q] = ne2;
-                b3[q] = nw2;
-            }
-            if (in2) {
-                oa[k2 - s0] = o2.a;
-                ob[k2 - s0] = o2.b;
-                oc[k2 - s0] = o2.c;
-            }
-        }
-        stage_mark(4);
-        // off-face links of each ring cell: all present neighbour values
-        // requested at once, summed in link order
-        for (int q = tid; q < nr; q += bs) {
-            int4 o0, o1;
-            float4 w0v, w1v;
-            A vc;
-            if (q == tid) {
-                o0 = fo0;
-                o1 = fo1;
-                w0v = fw0;
-                w1v = fw1;
-                vc = fvc;
-            } else {
-                o0 = __ldg(rn4 + 2 * q);
-                o1 = __ldg(rn4 + 2 * q + 1);
-                w0v = __ldg(rw4 + 2 * q);
-                w1v = __ldg(rw4 + 2 * q + 1);
-                int f, i, j;
-                ring_cell_of_rank(r0 + q, N, nring, f, i, j);
-                Own none;
-                vc = load((f * N + j) * N + i, false, none);
-            }
-            const int o[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
-            const float w[8] = {w0v.x, w0v.y, w0v.z, w0v.w, w1v.x, w1v.y, w1v.z, w1v.w};
-            A v[8];
+// The first taps of this thread's first row of an operator: they do not change
+// from cycle to cycle, so they are read before the grid barrier that the
+// operator's input waits for.
+constexpr int kPre = 8;
+struct Taps {
+    int2 q[kPre];
+    int len;
+};
+__device__ __forceinline__ void sp_prefetch(const SparseOp &op, Taps &T) {
+    const int total = op.rows;
+    const int e0 = min(32 * vwarp(), (total - 1) & ~31), e = min(e0 + (int)(threadIdx.x & 31), total - 1);
+    T.len = __ldg(op.glen + (e0 >> 5));
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                Own none;
-                v[k] = o[k] >= 0 ? load(o[k], false, none) : vc;
-            }
-            A t = 0;
+    for (int u = 0; u < kPre; u++)
+        T.q[u] = u < op.steps ? __ldg(op.tap + (size_t)u * total + e) : make_int2(0, 0);
+}
+
+// put(row, sum over the row's taps of weight * get(index)), rows spread over
+// the virtual grid, one thread per row; T: sp_prefetch's.  Bound by latency (a
+// gather round per kPre taps, the next taps in flight beside it).
+template <bool MP, class Get, class Put>
+__device__ __forceinline__ void sp_rows(const SparseOp &op, Taps &T, Get get, Put put) {
+    const int total = op.rows, lane = threadIdx.x & 31, steps = op.steps;
+    const int stride = 32 * vwarps();
+    const int2 *const tap = op.tap;
+    int e0 = 32 * vwarp(), s = 0;
+    DotAcc<MP> acc;
+#pragma unroll 1
+    while (e0 < total) {
+        float x[kPre];
 #pragma unroll
-            for (int k = 0; k < 8; k++)
-                if (o[k] >= 0) t += (A)w[k] * (vc - v[k]);
-            rs[q] = t;
+        for (int u = 0; u < kPre; u++) x[u] = get(T.q[u].x);
+        // the next taps: of this row, or the first of the thread's next row
+        // (rows past the end repeat the last element; their sums are unused)
+        const bool more = s + kPre < T.len;
+        const int en = more ? e0 : e0 + stride, sn = more ? s + kPre : 0;
+        Taps W;
+        W.len = T.len;
+        if (en < total) {
+            const int2 *t = tap + min(en + lane, total - 1);
+            if (!more) W.len = __ldg(op.glen + (en >> 5));
+#pragma unroll
+            for (int u = 0; u < kPre; u++)
+                W.q[u] = sn + u < steps ? __ldg(t + (size_t)(sn + u) * total) : make_int2(T.q[0].x, 0);
         }
-        __syncthreads();
-        stage_mark(2);
-        // two independent cells in flight per thread: one cell's dependent
-        // chain (shared loads, sum, conversions) leaves the issue slots idle
-        // with 16 warps per SM
-#pragma unroll 2
-        for (int c = s0 + tid; c < s1; c += bs) {
-            Own o;
-            o.a = oa[c - s0];
-            o.b = ob[c - s0];
-            o.c = oc[c - s0];
-            cell(c, bx - w0, b0 - w0, b1 - w0, b2 - w0, b3 - w0, rs, r0, o);
+#pragma unroll
+        for (int u = 0; u < kPre; u++) acc.add(__int_as_float(T.q[u].y), x[u]);
+        if (!more) {
+            if (e0 + lane < total) put(e0 + lane, (float)acc.a);
+            acc = DotAcc<MP>();
         }
-        __syncthreads();
-        stage_mark(3);
-        s0 = s1;
+        T = W;
+        e0 = en;
+        s = sn;
     }
 }
 
-#define STAGED_ARGS                                                                                            \
-    const typename Prec<MP>::A *x, const typename Prec<MP>::A *wE, const typename Prec<MP>::A *wN,           \
-        const typename Prec<MP>::A *wNE, const typename Prec<MP>::A *wNW, const typename Prec<MP>::A *rsum, \
-        int r0, Own o
-#define APPLY(S, c, xc) apply_k_smem(S, c, xc, x, wE, wN, wNE, wNW, rsum, r0)
+// ---- setup: the coarse levels inside one block -------------------------------
 
-// The pre-smoothed iterate from 0 at cell k: w D^-1 b (as stored).
-template <bool MP>
-__device__ __forceinline__ float presmooth_x(const LevelDev &L, int k, float b) {
-    if (MP) return as_stored<true>(0.8f * __ldg(L.dinv + k) * b);
-    return (float)(kOmegaJ * __ldg(L.dinv + k) * b);
+// (R r_fine) at coarse cell c (the CSR row of R = P^T).
+__device__ __forceinline__ float restrict_value(const LevelDev &F, const float *r, int c) {
+    const int k0 = __ldg(F.rstart + c), k1 = __ldg(F.rstart + c + 1);
+    double acc = 0;
+    for (int k = k0; k < k1; k++) acc += (double)(__ldg(F.rw + k) * r[__ldg(F.ridx + k)]);
+    return (float)acc;
 }
 
-// (R r_fine) at coarse cell c (times 1/4 in the mixed V-cycle).  Interior
-// coarse cells gather their 4x4 fine window in the CSR row order (fine index
-// ascending) with the P weights; the others use the CSR rows.
-template <bool MP>
-__device__ __forceinline__ float restrict_value(const LevelDev &F, const LevelDev &C, int c) {
-    using A = typename Prec<MP>::A;
-    const int Nc = C.S.N, Nf = F.S.N;
-    const auto *r = lv<MP>(F.r);
-    int f, I, J;
-    cell_fij(C.S, c, f, I, J);
-    A acc = 0;
-    if (F.structured && I >= 1 && J >= 1 && I + 2 <= Nc && J + 2 <= Nc) {
-        const int base = (f * Nf + 2 * J - 1) * Nf + 2 * I - 1;
-        const int nc = C.S.n;
-        float wv[16], rv[16];
-#pragma unroll
-        for (int dj = 0; dj < 4; dj++)
-#pragma unroll
-            for (int di = 0; di < 4; di++) {
-                const int i = base + dj * Nf + di;
-                wv[dj * 4 + di] = __ldg(F.rw16 + (dj * 4 + di) * nc + c);
-                rv[dj * 4 + di] = ldv(r, i);
-            }
-#pragma unroll
-        for (int q = 0; q < 16; q++) acc += (A)(wv[q] * rv[q]);
-    } else {
-        const int k0 = __ldg(F.rstart + c), k1 = __ldg(F.rstart + c + 1);
-        for (int k = k0; k < k1; k++) acc += (A)(__ldg(F.rw + k) * ldv(r, __ldg(F.ridx + k)));
-    }
-    return (float)acc * restrict_scale<MP>();
-}
-template <bool MP>
-__device__ __forceinline__ void restrict_cell(const LevelDev &F, const LevelDev &C, int c) {
-    stv(lv<MP>(C.b), c, restrict_value<MP>(F, C, c));
-}
-
-// x_fine + P xo_coarse (times 4 in the mixed V-cycle) at fine cell i.
-// Interior fine cells compute their 2x2 coarse taps.
-template <bool MP>
-__device__ __forceinline__ float prolong_value(const LevelDev &F, const LevelDev &C, int i) {
-    const int Nf = F.S.N, Nc = C.S.N;
-    (void)Nf;
+// x + P xc at fine cell i.
+__device__ __forceinline__ float prolong_value(const LevelDev &F, const float *x, const float *xc, int i) {
     const float4 w = __ldg(reinterpret_cast<const float4 *>(F.pw) + i);
-    const auto *xc = lv<MP>(C.xo);
-    int t0, t1, t2, t3;
-    int f, fi, fj;
-    cell_fij(F.S, i, f, fi, fj);
-    const int I0 = (fi - 1) >> 1, J0 = (fj - 1) >> 1;
-    if (F.structured && I0 >= 0 && J0 >= 0 && I0 + 1 < Nc && J0 + 1 < Nc) {
-        t0 = (f * Nc + J0) * Nc + I0;
-        t1 = t0 + 1;
-        t2 = t0 + Nc;
-        t3 = t0 + Nc + 1;
-    } else {
-        const int4 t = __ldg(reinterpret_cast<const int4 *>(F.ptap) + i);
-        t0 = t.x;
-        t1 = t.y;
-        t2 = t.z;
-        t3 = t.w;
-    }
-    const float s = w.x * ldv(xc, t0) + w.y * ldv(xc, t1) + w.z * ldv(xc, t2) + w.w * ldv(xc, t3);
-    if (MP) return ldv(lv<MP>(F.x), i) + 4.0f * s;
-    return ldv(lv<MP>(F.x), i) + (float)(kCorrScale * s);
+    const int4 t = __ldg(reinterpret_cast<const int4 *>(F.ptap) + i);
+    const float s = w.x * xc[t.x] + w.y * xc[t.y] + w.z * xc[t.z] + w.w * xc[t.w];
+    return x[i] + (float)(kCorrScale * s);
 }
 
-// Pre-smooth of a level from x = 0 with right-hand side bscale * b:
-// x = w D^-1 b, r = b - K x.
-template <bool MP, class TB>
-__device__ __forceinline__ void phase_presmooth(const LevelDev &L, const TB *b, float bscale, double *buf) {
-    using A = typename Prec<MP>::A;
-    auto load = [&](int k, bool mine, Own &o) -> A {
-        const float bk = MP ? ldv(b, k) * bscale : ldv(b, k);
-        if (mine) o.a = bk;
-        return (A)presmooth_x<MP>(L, k, bk);
-    };
-    auto commit = [&](int, const Own &) {};
-    auto *lx = lv<MP>(L.x);
-    auto *lr = lv<MP>(L.r);
-    staged<MP>(L.S, buf, load, commit, [&](int c, STAGED_ARGS) {
-        const float bc = o.a;
-        const float xc = (float)x[c];  // = presmooth_x(L, c, bc)
-        const A kx = APPLY(L.S, c, (A)xc);
-        stv(lx, c, xc);
-        stv(lr, c, (float)(bc - kx));
-    });
+// One damped-Jacobi sweep of src at cell c.
+__device__ __forceinline__ float jacobi_cell(const StencilDev &S, const float *dinv, float bc, const float *src,
+                                             int c) {
+    auto X = [&](int k) -> double { return (double)src[k]; };
+    const float xc = src[c];
+    const float rc = (float)(bc - apply_k(S, c, (double)xc, X));
+    return xc + (float)(kOmegaJ * __ldg(dinv + c) * rc);
 }
 
-// Prolongation C -> L fused with L's post-smooth: x = x_L + P xo_C is formed on
-// the fly over the staged window (never stored), then xo = x + w D^-1 (b - K x)
-// with b = bscale * b_in, stored as oscale * xo; returns sum dotr . (oscale xo)
-// in s (and sum dotr . zold in so) when dotr != nullptr.  Same arithmetic as a
-// separate prolongation pass followed by the post-smooth, one grid barrier fewer.
-template <bool MP, class TB, class TO>
-__device__ __forceinline__ void phase_prolong_postsmooth(const LevelDev &L, const LevelDev &C, const TB *b,
-                                                         float bscale, TO *xo, float oscale, const float *dotr,
-                                                         const float *zold, double &s, double &so, double *buf) {
-    using A = typename Prec<MP>::A;
-    auto load = [&](int k, bool mine, Own &o) -> A {
-        if (mine) {
-            o.a = MP ? ldv(b, k) * bscale : ldv(b, k);
-            o.b = __ldg(L.dinv + k);
-            o.c = dotr ? dotr[k] : 0.f;
-            if (MP) o.d = zold ? zold[k] : 0.f;
-        }
-        return (A)prolong_value<MP>(L, C, k);
-    };
-    double so_ = 0;
-    auto commit = [&](int, const Own &o) {
-        if (MP) so_ += (double)o.c * o.d;
-    };
-    staged<MP>(L.S, buf, load, commit, [&](int c, STAGED_ARGS) {
-        const float xc = (float)x[c];
-        const float rc = (float)(o.a - APPLY(L.S, c, (A)xc));
-        float out;
-        if (MP)
-            out = (xc + 0.8f * o.b * rc) * oscale;
-        else
-            out = xc + (float)(kOmegaJ * o.b * rc);
-        s += (double)o.c * stv_get(xo, c, out);
-    });
-    so = so_;
-}
-
-// One damped-Jacobi sweep src -> dst with per-link conversions (small levels).
-template <bool MP>
-__device__ __forceinline__ float jacobi_cell(const StencilDev &S, const float *dinv, const typename Prec<MP>::V *b,
-                                             const typename Prec<MP>::V *src, typename Prec<MP>::V *dst, int c) {
-    auto X = [&](int k) -> double { return (double)ldv(src, k); };
-    float xc = ldv(src, c);
-    float rc = (float)(ldv(b, c) - apply_k(S, c, (double)xc, X));
-    float out = xc + (float)(kOmegaJ * __ldg(dinv + c) * rc);
-    stv(dst, c, out);
-    return out;
-}
-
-// ---- the coarse levels inside one block (setup of the dense map, fallback) --
-// Always FP32 vectors in shared memory with the plain arithmetic: the V-cycle
-// of these levels maps b_l0 to xo_l0 the same way in both precisions (the
-// mixed transfer factors 1/4 and 4 cancel within it).
+// The V-cycle of the coarse levels on FP32 vectors in shared memory (the dense
+// map's columns; the transfers' factors 1/4 and 4 cancel within it).
 
 struct SmemLevel {
     float *x, *xo, *b, *r;
@@ -551,7 +551,7 @@ __device__ __forceinline__ void coarsest_smem(const LevelDev &L, const SmemLevel
         }
     } else {
         for (int s = 0; s < sweeps; s++) {
-            BLOCK_LOOP(c, n) jacobi_cell<false>(L.S, L.dinv, V.b, src, dst, c);
+            BLOCK_LOOP(c, n) dst[c] = jacobi_cell(L.S, L.dinv, V.b[c], src, c);
             __syncthreads();
             float *t = src;
             src = dst;
@@ -565,17 +565,12 @@ __device__ __forceinline__ void coarsest_smem(const LevelDev &L, const SmemLevel
 }
 
 // Levels l0..nlev-1 of the V-cycle inside this block, on vectors in shared
-// memory.  b of level l0 is lv[l0].b on entry; xo of level l0 is left in
-// lv[l0].xo.  Always inlined (with coarsest_smem): a call that takes the
-// solve's parameters by reference makes the compiler copy the whole
-// parameter block of the kernel to local memory, and every parameter read of
-// every phase then goes through it (measured: the solve 40 % slower).
+// memory.  b of level l0 is lv_[l0].b on entry; xo of level l0 is left in
+// lv_[l0].xo.
 __device__ __forceinline__ void vcycle_block_smem(const SolveParams &P, int l0, SmemLevel *lv_) {
     const int last = P.nlev - 1;
     for (int l = l0; l < last; l++) {
-        LevelDev L = P.L[l];
-        L.x = lv_[l].x;
-        L.r = lv_[l].r;
+        const LevelDev &L = P.L[l];
         const float *b = lv_[l].b;
         float *lx = lv_[l].x, *lr = lv_[l].r;
         BLOCK_LOOP(c, L.S.n) {
@@ -587,162 +582,223 @@ __device__ __forceinline__ void vcycle_block_smem(const SolveParams &P, int l0, 
             lr[c] = (float)(bc - kx);
         }
         __syncthreads();
-        LevelDev C = P.L[l + 1];
-        C.b = lv_[l + 1].b;
-        BLOCK_LOOP(c, C.S.n) restrict_cell<false>(L, C, c);
+        BLOCK_LOOP(c, P.L[l + 1].S.n) lv_[l + 1].b[c] = restrict_value(L, lr, c);
         __syncthreads();
     }
     coarsest_smem(P.L[last], lv_[last], P.coarse_sweeps);
     for (int l = last - 1; l >= l0; l--) {
-        LevelDev L = P.L[l];
-        L.x = lv_[l].x;
-        LevelDev C = P.L[l + 1];
-        C.xo = lv_[l + 1].xo;
-        BLOCK_LOOP(i, L.S.n) lv_[l].x[i] = prolong_value<false>(L, C, i);
+        const LevelDev &L = P.L[l];
+        const float *xc = lv_[l + 1].xo;
+        BLOCK_LOOP(i, L.S.n) lv_[l].x[i] = prolong_value(L, lv_[l].x, xc, i);
         __syncthreads();
-        BLOCK_LOOP(c, L.S.n) jacobi_cell<false>(L.S, L.dinv, lv_[l].b, lv_[l].x, lv_[l].xo, c);
+        BLOCK_LOOP(c, L.S.n) lv_[l].xo[c] = jacobi_cell(L.S, L.dinv, lv_[l].b[c], lv_[l].x, c);
         __syncthreads();
     }
 }
 
-// ---- the V-cycle after level 0's pre-smooth --------------------------------
+// ---- the coarse end of the V-cycle ------------------------------------------
 
-// The rest of z = V(r) once level 0's pre-smooth (x, r of level 0) is complete
-// and visible; the V-cycle ran on s0 * r (s0 = 1 in the plain solve).  Ends
-// with rz = r . z (and, mixed, r . z_prev) published; returns false on abort.
-template <bool MP>
-__device__ bool vcycle_rest(const SolveParams &P, const float *r, float s0, float *z, const float *zold,
-                            double *s_red, double *buf, float *smem) {
-    const int G = P.nlev_grid;
-    // down
-    for (int l = 0; l < G; l++) {
-        const LevelDev &L = P.L[l];
-        if (l > 0) {
-            phase_presmooth<MP>(L, lv<MP>(L.b), 1.0f, buf);
-            trace_mark(P, 100 + l);
-            SYNC_OR(return false);
-        }
-        GRID_LOOP(c, P.L[l + 1].S.n) restrict_cell<MP>(L, P.L[l + 1], c);
-        trace_mark(P, 300 + l);
-        SYNC_OR(return false);
-    }
-    // below the grid levels: the dense map, or block 0
-    if (P.dense) {
-        const LevelDev &C = P.L[G];
-        const auto *cb = lv<MP>(C.b);
-        auto *cx = lv<MP>(C.xo);
-        const int nd = P.nd, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int gw = vb() * (blockDim.x >> 5) + warp, nw = vnb() * (blockDim.x >> 5);
-        for (int row = gw; row < nd; row += nw) {
-            const double *d = P.dense + (size_t)row * nd;
-            double acc = 0;
-            for (int j = lane; j < nd; j += 32) acc += __ldg(d + j) * (double)ldv(cb, j);
+// put(row, sum_j D[row][j] b[j]) for every row of the dense map, two adjacent
+// warps per row, FP64 sums; get4(j) gives b[j..j+3] (anything past the end: the
+// map's padding columns are 0).  Bound by reading D from L2 (9.4 MB at nd =
+// 1536, 56 MB at 3750): 16-byte loads, the first kDensePre of a lane before the
+// grid barrier.  D holds FP32 values (the V-cycle it was built from works on
+// FP32 vectors), so FP32 storage loses nothing against FP64 and halves the
+// bytes.
+constexpr int kDensePre = 6;
+struct DenseTaps {
+    float4 w[kDensePre];
+};
+__device__ __forceinline__ void dense_prefetch(DenseTaps &T) {
+    const int ld4 = sP.ld >> 2, h4 = (ld4 + 1) >> 1, lane = threadIdx.x & 31;
+    const int part = min(vb() * ((int)blockDim.x >> 5) + (int)(threadIdx.x >> 5), 2 * sP.nd - 1);
+    const int j0 = (part & 1) * h4, j1 = min(ld4, j0 + h4);
+    const float4 *d = reinterpret_cast<const float4 *>(sP.dense) + (size_t)(part >> 1) * ld4;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) stv(cx, row, (float)acc);
+    for (int u = 0; u < kDensePre; u++)
+        T.w[u] = j0 + lane + 32 * u < j1 ? __ldg(d + j0 + lane + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+template <class Get4, class Put>
+__device__ __forceinline__ void dense_rows(const DenseTaps &T, Get4 get4, Put put) {
+    __shared__ double s_half[32];
+    const int nd = sP.nd, ld4 = sP.ld >> 2, h4 = (ld4 + 1) >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nw = (int)blockDim.x >> 5;  // even
+    bool first = true;
+#pragma unroll 1
+    for (int base = vb() * nw; base < 2 * nd; base += vnb() * nw) {
+        const int part = min(base + warp, 2 * nd - 1);
+        const int j1 = min(ld4, ((part & 1) + 1) * h4);
+        const float4 *d = reinterpret_cast<const float4 *>(sP.dense) + (size_t)(part >> 1) * ld4;
+        double v = 0;
+        auto add = [&](float4 w, float4 b) {
+            v += (double)w.x * (double)b.x;
+            v += (double)w.y * (double)b.y;
+            v += (double)w.z * (double)b.z;
+            v += (double)w.w * (double)b.w;
+        };
+        int j = (part & 1) * h4 + lane;
+        if (first) {
+#pragma unroll
+            for (int u = 0; u < kDensePre; u++) add(T.w[u], get4(4 * min(j + 32 * u, ld4 - 1)));
+            j += 32 * kDensePre;
         }
-        trace_mark(P, 500);
-        SYNC_OR(return false);
-    } else if (!P.coarse_on_grid) {
-        if (vb() == 0) {
-            SmemLevel lvs[kMaxLev];
-            carve_smem(P, G, smem, lvs);
-            const auto *gb = lv<MP>(P.L[G].b);
-            BLOCK_LOOP(c, P.L[G].S.n) lvs[G].b[c] = ldv(gb, c);
-            __syncthreads();
-            vcycle_block_smem(P, G, lvs);
-            auto *gx = lv<MP>(P.L[G].xo);
-            BLOCK_LOOP(c, P.L[G].S.n) stv(gx, c, lvs[G].xo[c]);
-        }
-        trace_mark(P, 500);
-        SYNC_OR(return false);
-    } else {
-        // the coarsest level is large (nlev_grid == nlev - 1): sweep it grid-wide
-        const LevelDev &L = P.L[P.nlev - 1];
-        auto *lx = lv<MP>(L.x), *lxo = lv<MP>(L.xo);
-        const auto *lb = lv<MP>(L.b);
-        GRID_LOOP(c, L.S.n) stv(lx, c, 0.f);
-        SYNC_OR(return false);
-        auto *src = lx, *dst = lxo;
-        for (int s = 0; s < P.coarse_sweeps; s++) {
-            GRID_LOOP(c, L.S.n) jacobi_cell<MP>(L.S, L.dinv, lb, src, dst, c);
-            SYNC_OR(return false);
-            auto *t = src;
-            src = dst;
-            dst = t;
-        }
-        if (src != lxo) {
-            GRID_LOOP(c, L.S.n) lxo[c] = src[c];
-            SYNC_OR(return false);
-        }
+        first = false;
+#pragma unroll 4
+        for (; j < j1; j += 32) add(__ldg(d + j), get4(4 * j));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) s_half[warp] = v;
+        __syncthreads();
+        if (lane == 0 && !(warp & 1) && base + warp < 2 * nd) put(part >> 1, s_half[warp] + s_half[warp + 1]);
+        __syncthreads();
     }
-    // up: prolongation fused with each grid level's post-smooth
-    for (int l = G - 1; l >= 0; l--) {
-        const LevelDev &L = P.L[l];
-        double s = 0, so = 0;
-        if (l > 0) {
-            phase_prolong_postsmooth<MP>(L, P.L[l + 1], lv<MP>(L.b), 1.0f, lv<MP>(L.xo), 1.0f, nullptr, nullptr, s, so,
-                                         buf);
-            trace_mark(P, 900 + l);
-            SYNC_OR(return false);
-        } else {
-            phase_prolong_postsmooth<MP>(L, P.L[1], r, s0, z, 1.0f / s0, r, zold, s, so, buf);
-            put_partial(P, RED_RZ, s, s_red);
-            if (MP) put_partial(P, RED_RZO, so, s_red);
-            trace_mark(P, 900);
-            SYNC_OR(return false);
-        }
-    }
-    return true;
 }
 
-// z = V(r) for a single-level hierarchy (level 0 is the coarsest grid); the
-// sweeps run on s0 * r (s0 = 1 in the plain solve).
-template <bool MP>
-__device__ bool single_level(const SolveParams &P, const float *r, float s0, float *z, const float *zold,
-                             double *s_red, float *smem) {
-    const LevelDev &L = P.L[0];
-    auto *lx = lv<MP>(L.x), *lxo = lv<MP>(L.xo);
-    auto *lb = lv<MP>(L.b);
-    if (!P.coarse_on_grid) {
-        if (vb() == 0) {
-            SmemLevel lvs[kMaxLev];
-            carve_smem(P, 0, smem, lvs);
-            BLOCK_LOOP(c, L.S.n) lvs[0].b[c] = r[c];
-            __syncthreads();
-            coarsest_smem(L, lvs[0], P.coarse_sweeps);
-            BLOCK_LOOP(c, L.S.n) stv(lxo, c, MP ? lvs[0].xo[c] * s0 : lvs[0].xo[c]);
+// The coarsest level's damped-Jacobi sweeps from 0, grid-wide, in FP32
+// (upstream src/fluid.c:118-137), for a level too large for the dense map.
+// With a thread for every cell its links stay in registers, so that a sweep is
+// one gather round and one grid barrier.  Returns the buffer that holds the
+// result (read at the own cell only), or nullptr on abort.
+template <bool MP, class GetB>
+__device__ __forceinline__ const float *coarse_sweeps(const LevelDev &L, GetB getb) {
+    const int n = L.S.n;
+    float *src = sP.sw0, *dst = sP.sw1;
+    if (n <= vnb() * (int)blockDim.x) {
+        const int c = vb() * blockDim.x + threadIdx.x;
+        int nb[kMaxNb];
+        float wv[kMaxNb], bc = 0.f, xc = 0.f;
+        double od = 0;
+        if (c < n) {
+            cell_links(L.S, c, nb, wv);
+            bc = getb(c);
+            od = kOmegaJ * __ldg(L.dinv + c);
+            xc = as_stored<MP>((float)(od * bc));  // the first sweep
+            src[c] = xc;
         }
-    } else {
-        GRID_LOOP(c, L.S.n) {
-            stv(lx, c, 0.f);
-            stv(lb, c, MP ? r[c] * s0 : r[c]);
-        }
-        SYNC_OR(return false);
-        auto *src = lx, *dst = lxo;
-        for (int s = 0; s < P.coarse_sweeps; s++) {
-            GRID_LOOP(c, L.S.n) jacobi_cell<MP>(L.S, L.dinv, lb, src, dst, c);
-            SYNC_OR(return false);
-            auto *t = src;
+#pragma unroll 1
+        for (int s = 1; s < sP.coarse_sweeps; s++) {
+            if (!vsync(0, 0, 0)) return nullptr;
+            if (c < n) {
+                float v[kMaxNb];
+#pragma unroll
+                for (int k = 0; k < kMaxNb; k++) v[k] = src[nb[k]];
+                double acc = 0;
+#pragma unroll
+                for (int k = 0; k < kMaxNb; k++) acc += (double)wv[k] * ((double)xc - (double)v[k]);
+                const float rc = (float)(bc - acc);
+                xc = as_stored<MP>(xc + (float)(od * rc));
+                dst[c] = xc;
+            }
+            float *t = src;
             src = dst;
             dst = t;
         }
-        if (src != lxo) {
-            GRID_LOOP(c, L.S.n) lxo[c] = src[c];
+        return src;
+    }
+    GRID_LOOP(c, n) src[c] = as_stored<MP>((float)(kOmegaJ * __ldg(L.dinv + c) * getb(c)));
+    for (int s = 1; s < sP.coarse_sweeps; s++) {
+        if (!vsync(0, 0, 0)) return nullptr;
+        GRID_LOOP(c, n) dst[c] = as_stored<MP>(jacobi_cell(L.S, L.dinv, getb(c), src, c));
+        float *t = src;
+        src = dst;
+        dst = t;
+    }
+    return src;
+}
+
+// ---- the grid levels of the V-cycle ------------------------------------------
+
+// The pre-smoothed iterate from 0 at cell k: w D^-1 b (as stored).
+template <bool MP>
+__device__ __forceinline__ float presmooth_x(float dinv, float b) {
+    if (MP) return as_stored<true>(0.8f * dinv * b);
+    return (float)(kOmegaJ * dinv * b);
+}
+
+// The restriction's operands of this thread's first coarse cell and ring row,
+// read before the grid barrier.
+struct RestrictPre {
+    float w[16];
+    Taps t;
+};
+__device__ __forceinline__ void restrict_prefetch(int l, RestrictPre &R) {
+    const int nc = sP.L[l + 1].S.n, c = min(s_range[l + 1][0] + (int)threadIdx.x, nc - 1);
+    const float *rw16 = sP.L[l].rw16;
+    if (rw16) {
+#pragma unroll
+        for (int q = 0; q < 16; q++) R.w[q] = __ldg(rw16 + (size_t)q * nc + c);
+    }
+    sp_prefetch(sP.L[l].rst, R.t);
+}
+
+// b of level l + 1 = R r of level l (times 1/4 in the mixed V-cycle).  Interior
+// coarse cells gather their 4 x 4 fine window with the weights of rw16
+// (coarse-major), in the row order of R (fine index ascending); the others (the
+// ring of the coarse level, or every cell when the pattern does not hold) are
+// sparse rows.
+template <bool MP>
+__device__ __forceinline__ void restrict_phase(int l, RestrictPre &R) {
+    using A = typename Prec<MP>::A;
+    const LevelDev &F = sP.L[l], &Cl = sP.L[l + 1];
+    const StencilDev &C = Cl.S;
+    const int Nf = F.S.N, Nc = C.N, nc = C.n;
+    const auto *r = lv<MP>(F.r);
+    auto *b = lv<MP>(Cl.b);
+    const float *rw16 = F.rw16;
+    const float scale = MP ? 0.25f : 1.0f;
+    sp_rows<MP>(F.rst, R.t, [&](int k) { return ldv(r, k); }, [&](int row, float v) {
+        int c = row;
+        if (rw16) {
+            int f, i, j;
+            ring_cell_of_rank(row, Nc, C.nring, f, i, j);
+            c = (f * Nc + j) * Nc + i;
         }
+        stv(b, c, v * scale);
+    });
+    if (!rw16) return;
+    bool first = true;
+#pragma unroll 1
+    for (int c = s_range[l + 1][0] + (int)threadIdx.x; c < s_range[l + 1][1]; c += blockDim.x) {
+        int f, I, J;
+        cell_fij(C, c, f, I, J);
+        if (I >= 1 && J >= 1 && I + 2 <= Nc && J + 2 <= Nc) {
+            const int base = (f * Nf + 2 * J - 1) * Nf + 2 * I - 1;
+            float x[16];
+#pragma unroll
+            for (int q = 0; q < 16; q++) x[q] = ldv(r, base + (q >> 2) * Nf + (q & 3));
+            if (!first) {
+#pragma unroll
+                for (int q = 0; q < 16; q++) R.w[q] = __ldg(rw16 + (size_t)q * nc + c);
+            }
+            DotAcc<MP> acc;
+#pragma unroll
+            for (int q = 0; q < 16; q++) acc.add(R.w[q], x[q]);
+            stv(b, c, (float)acc.a * scale);
+        }
+        first = false;
     }
-    SYNC_OR(return false);
-    double s = 0, so = 0;
-    const float inv = 1.0f / s0;
-    GRID_LOOP(c, L.S.n) {
-        if (zold) so += (double)r[c] * zold[c];
-        float zc = MP ? ldv(lxo, c) * inv : ldv(lxo, c);
-        z[c] = zc;
-        s += (double)r[c] * zc;
+}
+
+// x + P xo (times 4 in the mixed V-cycle) of level l at cell k, x its
+// pre-smoothed iterate.  Inside a face the four coarse taps follow from the
+// cell's indices (where rw16 says the pattern holds).
+template <bool MP>
+__device__ __forceinline__ float prolong(const LevelDev &L, int Nc, const typename Prec<MP>::V *xc, int k, float b) {
+    const float4 w = __ldg(reinterpret_cast<const float4 *>(L.pw) + k);
+    const float x = presmooth_x<MP>(__ldg(L.dinv + k), b);
+    int f, i, j;
+    cell_fij(L.S, k, f, i, j);
+    int t0 = (f * Nc + ((j - 1) >> 1)) * Nc + ((i - 1) >> 1), t1 = t0 + 1, t2 = t0 + Nc, t3 = t2 + 1;
+    if (!L.rw16 || i == 0 || j == 0 || i == L.S.N - 1 || j == L.S.N - 1) {
+        const int4 t = __ldg(reinterpret_cast<const int4 *>(L.ptap) + k);
+        t0 = t.x;
+        t1 = t.y;
+        t2 = t.z;
+        t3 = t.w;
     }
-    put_partial(P, RED_RZ, s, s_red);
-    if (MP) put_partial(P, RED_RZO, so, s_red);
-    return vsync(P);
+    const float s = w.x * ldv(xc, t0) + w.y * ldv(xc, t1) + w.z * ldv(xc, t2) + w.w * ldv(xc, t3);
+    if (MP) return x + 4.0f * s;
+    return x + (float)(kCorrScale * s);
 }
 
 // Power of two that brings a residual of squared norm rr over n cells to an
@@ -754,290 +810,364 @@ __device__ __forceinline__ float vscale(double rr, int n) {
     return ldexpf(1.0f, max(-100, min(100, -4 - e)));
 }
 
-// The whole solve for the SolveParams of this block's planet, on the block's
-// virtual grid (vb(), vnb()).
+// The whole solve of this block's planet (sP) on the block's virtual grid.
 template <bool MP>
-__device__ __forceinline__ void pcg_body(const SolveParams &P) {
-    __shared__ Red sh;
-    extern __shared__ __align__(16) unsigned char dyn[];
-    double *buf = reinterpret_cast<double *>(dyn);               // staged window
-    float *smem = reinterpret_cast<float *>(dyn + kStageBytes);  // block-0 levels
-    double *s_red = sh.v;
-    // the warp slots of warps this block does not have stay zero (ordered
-    // before the first read by the first block sum's barriers)
-    if (threadIdx.x < kRedBlock / 32) s_red[threadIdx.x] = 0.0;
+__device__ __forceinline__ void pcg_body() {
     using A = typename Prec<MP>::A;
-    const LevelDev &L0 = P.L[0];
-    const StencilDev &S0 = L0.S;
-    const int n = S0.n;
-    const bool mg = P.nlev >= 2;
-    const bool single = P.nlev == 1;
-    float *r = P.r, *rn = P.r2, *p = P.p, *pn = P.p2;
-    float *z = P.z, *zo = MP ? P.z2 : nullptr;  // mixed: z / z2 ping-pong (the previous z for the flexible beta)
-    double bb, rr, rz = 0, tol2, beta = 0, m2;
+    using V = typename Prec<MP>::V;
+    const int n = sP.L[0].S.n;
+    const bool mg = sP.nlev >= 2, single = sP.nlev == 1;
+    const int G = sP.nlev_grid;
+    float *r = sP.r, *rn = sP.r2, *p = sP.p, *pn = sP.p2;
+    float *z = sP.z, *zo = MP ? sP.z2 : nullptr;  // mixed: z / z2 ping-pong (the previous z for the flexible beta)
+    double bb = 0, rr = 0, rz = 0, tol2 = 0, beta = 0, m2;
     int it = 0, flags = 0;
-    bool first = true, ok = true;
+    bool init = true, ok = false;
     float s0 = 1.0f;
     const unsigned long long t_begin = threadIdx.x == 0 ? globaltimer_ns() : 0ull;
+    block_setup();
+    RingPre R;
+    ring_prefetch(0, R);
 
-    // zero-mean projection of omega (FP64 sum), upstream src/fluid.c:264-275
-    if (P.remove_mean) {
-        double s = 0;
-        GRID_LOOP(c, n) s += (double)__ldg(P.area + c) * P.omega[c];
-        put_partial(P, RED_MEAN, s, s_red);
-        SYNC_OR(goto aborted);
-        float m = (float)(get_total(P, RED_MEAN, s_red) / P.total_area);
-        GRID_LOOP(c, n) P.omega[c] -= m;  // read back below only at the own cell
-    }
-
-    // FP64 projection that makes the singular system consistent: the stored
-    // FP32 omega keeps a residual area-weighted mean m2 (the FP32 rounding of
-    // the subtracted mean); b = -A (omega - m2) is formed in FP64 so that
+    // zero-mean projection of omega (FP64 sum), upstream src/fluid.c:264-275,
+    // then the FP64 projection that makes the singular system consistent: the
+    // stored FP32 omega keeps a residual area-weighted mean m2 (the FP32 rounding
+    // of the subtracted mean); b = -A (omega - m2) is formed in FP64 so that
     // sum b = 0 to double precision.  Without it the constant mode of the
     // residual stays at the FP32 rounding level and CG diverges once the
     // residual reaches it.
-    {
+#pragma unroll 1
+    for (int pass = sP.remove_mean ? 0 : 1; pass < 2; pass++) {
+        const float *area = sP.area;
+        float *omega = sP.omega;
         double s = 0, sa = 0;
-        GRID_LOOP(c, n) {
-            double a = __ldg(P.area + c);
-            s += a * P.omega[c];
+#pragma unroll 4
+        OWN_LOOP(c) {
+            const double a = __ldg(area + c);
+            s += a * omega[c];
             sa += a;
         }
-        put_partial(P, RED_MEAN, s, s_red);
-        put_partial(P, RED_AREA, sa, s_red);
-        SYNC_OR(goto aborted);
-        m2 = get_total(P, RED_MEAN, s_red) / get_total(P, RED_AREA, s_red);
-    }
-
-    // r = b - K psi, b = -A (omega - m2)
-    {
-        double sb = 0, sr = 0;
-        const float *psi = P.psi;
-        auto load = [&](int k, bool mine, Own &o) -> A {
-            if (mine) {
-                o.a = P.omega[k];
-                o.b = __ldg(P.area + k);
-            }
-            return (A)psi[k];
-        };
-        auto commit = [&](int, const Own &) {};
-        staged<MP>(S0, buf, load, commit, [&](int c, STAGED_ARGS) {
-            double b = -(double)o.b * ((double)o.a - m2);
-            double ri = b - (double)APPLY(S0, c, x[c]);
-            r[c] = (float)ri;
-            sb += b * b;
-            sr += ri * ri;
-        });
-        put_partial(P, RED_BB, sb, s_red);
-        put_partial(P, RED_RR, sr, s_red);
-    }
-    SYNC_OR(goto aborted);
-    bb = get_total(P, RED_BB, s_red);
-    rr = get_total(P, RED_RR, s_red);
-    if (!isfinite(bb) || !isfinite(rr)) flags |= kSolveNonFinite;
-    if (bb == 0.0) {
-        GRID_LOOP(c, n) P.psi[c] = 0.f;
-        if (vb() == 0 && threadIdx.x == 0) {
-            P.res->iters = 0;
-            P.res->relres = 0;
-            P.res->status = 0;
-            P.res->r_final = 0;
-            P.res->flags = flags;
-            P.res->ns = globaltimer_ns() - t_begin;
-        }
-        return;
-    }
-    tol2 = P.tol * P.tol * bb;
-
-    // z = M^-1 r, rz
-    if (rr > tol2) {
-        if (mg) {
-            s0 = vscale<MP>(rr, n);
-            phase_presmooth<MP>(L0, r, s0, buf);
-            SYNC_OR(goto aborted);
-            ok = vcycle_rest<MP>(P, r, s0, z, nullptr, s_red, buf, smem);
-        } else if (single) {
-            s0 = vscale<MP>(rr, n);
-            ok = single_level<MP>(P, r, s0, z, nullptr, s_red, smem);
+        if (!vsync(2, s, sa)) goto done;
+        const double tot = s_total[0];
+        if (pass == 0) {
+            const float m = (float)(tot / sP.total_area);
+#pragma unroll 4
+            OWN_LOOP(c) omega[c] -= m;  // read back by the same thread before the next grid barrier
         } else {
-            double s = 0;
-            GRID_LOOP(c, n) {
-                float zc = __ldg(L0.dinv + c) * r[c];
-                z[c] = zc;
-                s += (double)r[c] * zc;
-            }
-            put_partial(P, RED_RZ, s, s_red);
-            ok = vsync(P);
+            m2 = tot / s_total[1];
         }
-        if (!ok) goto aborted;
-        rz = get_total(P, RED_RZ, s_red);
-        if (!isfinite(rz)) flags |= kSolveNonFinite;
     }
 
-    while (rr > tol2 && it < P.maxit) {
-        // p = z (first) or z + beta p;  Ap = K p;  pAp
+#pragma unroll 1
+    for (;;) {
+        RestrictPre T;
+        DenseTaps D;
+        double s = 0, s2 = 0;
+        // first r = b - K psi, b = -A (omega - m2); then p = z or z + beta p, Ap = K p
         {
-            const float *zz = z;
-            const float *po = p;
-            const bool fst = first;
+            const float *xa = init ? sP.psi : z;
+            const float *xb = p;
+            const bool comb = !init && it > 0;
             const double be = beta;
-            auto pnew = [&](int k) -> float { return fst ? zz[k] : (float)(zz[k] + be * po[k]); };
-            auto load = [&](int k, bool, Own &) -> A { return (A)pnew(k); };
-            auto commit = [&](int, const Own &) {};
-            double s = 0;
-            float *pw = pn, *ap = P.Ap;
-            staged<MP>(S0, buf, load, commit, [&](int c, STAGED_ARGS) {
-                const float pc = (float)x[c];
-                const A a = APPLY(S0, c, (A)pc);
-                pw[c] = pc;
-                ap[c] = (float)a;
-                s += (double)a * pc;
-            });
-            put_partial(P, RED_PAP, s, s_red);
-            float *t = p;
-            p = pn;
-            pn = t;
-            first = false;
+            float *xw = init ? r : pn, *ap = sP.Ap;
+            stencil_phase<MP>(0, R, [&](int k) { return comb ? (float)(xa[k] + be * xb[k]) : xa[k]; },
+                              [&](int c, float xc, A kx) {
+                                  if (init) {
+                                      const double b = -(double)__ldg(sP.area + c) * ((double)sP.omega[c] - m2);
+                                      const double ri = b - (double)kx;
+                                      xw[c] = (float)ri;
+                                      s2 += b * b;
+                                      s += ri * ri;
+                                  } else {
+                                      xw[c] = xc;
+                                      ap[c] = (float)kx;
+                                      s += (double)kx * xc;
+                                  }
+                              });
+            if (!init) {
+                pn = p;
+                p = xw;
+            }
         }
-        trace_mark(P, 10);
-        SYNC_OR(goto aborted);
-        trace_mark(P, 11);
-        {
-            double pAp = get_total(P, RED_PAP, s_red);
+        if (mg) ring_prefetch(0, R);
+        TRACE(10);
+        if (!vsync(init ? 2 : 1, s, s2)) goto done;
+        TRACE(11);
+        double alpha = 0;
+        if (init) {
+            rr = s_total[0];
+            bb = s_total[1];
+            if (!isfinite(bb) || !isfinite(rr)) flags |= kSolveNonFinite;
+            tol2 = sP.tol * sP.tol * bb;
+            if (bb == 0.0 || !(rr > tol2)) {
+                ok = true;
+                break;
+            }
+        } else {
+            const double pAp = s_total[0];
             if (!isfinite(pAp)) flags |= kSolveNonFinite;
             if (pAp <= 0) {
                 flags |= kSolveBreakdown;
+                ok = true;
                 break;
             }
-            const double alpha = rz / pAp;
-            const float *Ap = P.Ap;
-            const float *ro = r;
-            const float *pp = p;
-            double s = 0, sz = 0;
-            float *rw_ = rn;
-            if (mg) {
-                // the previous r's scale (the new r is not reduced yet)
-                s0 = vscale<MP>(rr, n);
-                const float sc = s0;
-                // psi += alpha p; r' = r - alpha Ap; level-0 pre-smooth of r'
-                auto rnew = [&](int k) -> float { return (float)(ro[k] - alpha * Ap[k]); };
-                // mine: r, Ap of the cell staged; p and psi kept for commit,
-                // which does psi += alpha p (nothing else reads psi)
-                auto load = [&](int k, bool mine, Own &o) -> A {
-                    if (mine) {
-                        o.a = ro[k];
-                        o.b = Ap[k];
-                        o.c = pp[k];
-                        o.d = P.psi[k];
-                    }
-                    return (A)presmooth_x<MP>(L0, k, MP ? rnew(k) * sc : rnew(k));
+            alpha = rz / pAp;
+        }
+        // psi += alpha p; r' = r - alpha Ap; the V-cycle's way down from r'
+        const float *ro = r, *Ap = sP.Ap;
+        s = s2 = 0;
+        if (mg || single) s0 = vscale<MP>(rr, n);  // the previous r's scale (the new r is not reduced yet)
+        if (mg) {
+#pragma unroll 1
+            for (int l = 0; l < G; l++) {
+                // pre-smooth from x = 0: x = w D^-1 b, r = b - K x
+                const LevelDev &L = sP.L[l];
+                const V *lb = lv<MP>(L.b);
+                V *lr = lv<MP>(L.r);
+                const float *dinv = L.dinv;
+                float *psi = sP.psi, *rw_ = rn;
+                auto getb = [&](int k) -> float {
+                    if (l > 0) return ldv(lb, k);
+                    const float v = init ? ro[k] : (float)(ro[k] - alpha * Ap[k]);
+                    return MP ? v * s0 : v;
                 };
-                auto commit = [&](int k, const Own &o) { P.psi[k] = o.d + (float)(alpha * o.c); };
-                auto *l0x = lv<MP>(L0.x);
-                auto *l0r = lv<MP>(L0.r);
-                staged<MP>(S0, buf, load, commit, [&](int c, STAGED_ARGS) {
-                    const double ri = o.a - alpha * o.b;
-                    const float rc = (float)ri;
-                    rw_[c] = rc;
-                    s += ri * ri;
-                    const float xc = (float)x[c];  // = presmooth_x(L0, c, rc * sc)
-                    const A kx = APPLY(S0, c, (A)xc);
-                    stv(l0x, c, xc);
-                    stv(l0r, c, (float)((MP ? rc * sc : rc) - kx));
-                });
-            } else {
-                GRID_LOOP(c, n) {
-                    P.psi[c] += (float)(alpha * pp[c]);
-                    double ri = ro[c] - alpha * Ap[c];
-                    float rc = (float)ri;
-                    rw_[c] = rc;
-                    s += ri * ri;
-                    if (!single) {
-                        float zc = __ldg(L0.dinv + c) * rc;
-                        z[c] = zc;
-                        sz += (double)rc * zc;
+                stencil_phase<MP>(l, R, [&](int k) { return presmooth_x<MP>(__ldg(dinv + k), getb(k)); },
+                                  [&](int c, float, A kx) {
+                                      if (l == 0 && !init) {
+                                          const double ri = ro[c] - alpha * Ap[c];
+                                          const float rc = (float)ri;
+                                          psi[c] += (float)(alpha * p[c]);
+                                          rw_[c] = rc;
+                                          s += ri * ri;
+                                          stv(lr, c, (float)((MP ? rc * s0 : rc) - kx));
+                                      } else {
+                                          stv(lr, c, (float)(getb(c) - kx));
+                                      }
+                                  });
+                restrict_prefetch(l, T);
+                TRACE(100 + l);
+                // |r'|^2 is read during the next phase (the test for convergence comes one phase late)
+                const bool res = l == 0 && !init;
+                if (!vsync(res ? 1 : 0, s, 0, true)) goto done;
+                restrict_phase<MP>(l, T);
+                if (l + 1 < G)
+                    ring_prefetch(l + 1, R);
+                else if (sP.dense)
+                    dense_prefetch(D);
+                TRACE(300 + l);
+                if (!vsync(0, 0, 0, false, res)) goto done;
+                if (res) {
+                    rn = r;
+                    r = rw_;
+                    it++;
+                    rr = s_late;
+                    if (!isfinite(rr)) flags |= kSolveNonFinite;
+                    if (rr <= tol2) {
+                        ok = true;
+                        break;
                     }
                 }
-                if (!single) put_partial(P, RED_RZ, sz, s_red);
             }
-            put_partial(P, RED_RR, s, s_red);
-            float *t = r;
-            r = rn;
-            rn = t;
+            if (ok) break;
+        } else {
+            float *rw_ = init ? r : rn;
+            OWN_LOOP(c) {
+                double ri = ro[c];
+                if (!init) {
+                    sP.psi[c] += (float)(alpha * p[c]);
+                    ri -= alpha * Ap[c];
+                    rw_[c] = (float)ri;
+                }
+                const float rc = (float)ri;
+                s += ri * ri;
+                if (!single) {
+                    const float zc = __ldg(sP.L[0].dinv + c) * rc;
+                    z[c] = zc;
+                    s2 += (double)rc * zc;
+                }
+            }
+            if (!init) {
+                rn = r;
+                r = rw_;
+            }
+            ring_prefetch(0, R);
+            if (!vsync(2, s, s2)) goto done;
+            if (!init) {
+                it++;
+                rr = s_total[0];
+                if (!isfinite(rr)) flags |= kSolveNonFinite;
+                if (rr <= tol2) {
+                    ok = true;
+                    break;
+                }
+                if (single) s0 = vscale<MP>(rr, n);
+            }
         }
-        it++;
-        trace_mark(P, 12);
-        SYNC_OR(goto aborted);
-        trace_mark(P, 13);
-        rr = get_total(P, RED_RR, s_red);
-        if (!isfinite(rr)) flags |= kSolveNonFinite;
-        if (rr <= tol2) break;
-        if (MP && (mg || single)) {  // the new z goes to the other buffer; zo keeps the previous one
+        // z = M^-1 r
+        const float *zold = nullptr;
+        if (MP && !init && (mg || single)) {  // the new z goes to the other buffer; zo keeps the previous one
             float *t = z;
             z = zo;
             zo = t;
+            zold = zo;
         }
-        if (mg)
-            ok = vcycle_rest<MP>(P, r, s0, z, MP ? zo : nullptr, s_red, buf, smem);
-        else if (single) {
-            s0 = vscale<MP>(rr, n);
-            ok = single_level<MP>(P, r, s0, z, MP ? zo : nullptr, s_red, smem);
+        if (mg || single) {
+            s = s2 = 0;
+            const float inv = 1.0f / s0;
+            auto finish = [&](int c, float v) {
+                const float rc = r[c], zc = MP ? v * inv : v;
+                z[c] = zc;
+                s += (double)rc * zc;
+                if (MP && zold) s2 += (double)rc * zold[c];
+            };
+            // the coarsest grid level: the dense map, or its sweeps
+            {
+                const LevelDev &L = sP.L[G];
+                const V *cb = lv<MP>(L.b);
+                V *cx = lv<MP>(L.xo);
+                auto getb = [&](int c) -> float {
+                    if (mg) return ldv(cb, c);
+                    return as_stored<MP>(MP ? r[c] * s0 : r[c]);
+                };
+                auto put = [&](int c, float v) {
+                    if (mg)
+                        stv(cx, c, v);
+                    else
+                        finish(c, as_stored<MP>(v));
+                };
+                if (sP.dense) {
+                    dense_rows(D, [&](int j) { return ldv4(cb + j); }, [&](int c, double v) { put(c, (float)v); });
+                } else if (!sP.coarse_on_grid) {
+                    // a single small level: block 0 sweeps r in shared memory
+                    if (vb() == 0) {
+                        SmemLevel lvl;
+                        lvl.x = s_win();
+                        lvl.xo = lvl.x + n;
+                        lvl.b = lvl.xo + n;
+                        BLOCK_LOOP(c, n) lvl.b[c] = r[c];
+                        __syncthreads();
+                        coarsest_smem(L, lvl, sP.coarse_sweeps);
+                        BLOCK_LOOP(c, n) put(c, MP ? lvl.xo[c] * s0 : lvl.xo[c]);
+                    }
+                } else {
+                    const float *x = coarse_sweeps<MP>(L, getb);
+                    if (!x) goto done;
+                    GRID_LOOP(c, L.S.n) put(c, x[c]);
+                }
+            }
+            if (mg) {
+                ring_prefetch(G - 1, R);
+                TRACE(500);
+                if (!vsync(0, 0, 0)) goto done;
+#pragma unroll 1
+                for (int l = G - 1;; l--) {
+                    // prolongation and post-smooth: x = x + P xo, then x + w D^-1 (b - K x)
+                    const LevelDev &L = sP.L[l];
+                    const V *lb = lv<MP>(L.b), *xc = lv<MP>(sP.L[l + 1].xo);
+                    V *lx = lv<MP>(L.xo);
+                    const int Nc = sP.L[l + 1].S.N;
+                    const float *dinv = L.dinv;
+                    auto getb = [&](int k) -> float {
+                        if (l > 0) return ldv(lb, k);
+                        return MP ? r[k] * s0 : r[k];
+                    };
+                    stencil_phase<MP>(l, R, [&](int k) { return prolong<MP>(L, Nc, xc, k, getb(k)); },
+                                      [&](int c, float x, A kx) {
+                                          const float rc = (float)(getb(c) - kx), d = __ldg(dinv + c);
+                                          const float v = MP ? x + 0.8f * d * rc : x + (float)(kOmegaJ * d * rc);
+                                          if (l > 0)
+                                              stv(lx, c, v);
+                                          else
+                                              finish(c, v);
+                                      });
+                    if (l == 0) break;
+                    ring_prefetch(l - 1, R);
+                    TRACE(900 + l);
+                    if (!vsync(0, 0, 0)) goto done;
+                }
+            }
+            ring_prefetch(0, R);
+            TRACE(900);
+            if (!vsync(MP ? 2 : 1, s, s2)) goto done;
         }
-        if (!ok) goto aborted;
         {
-            double rznew = get_total(P, RED_RZ, s_red);
+            const double rznew = mg || single ? s_total[0] : s_total[1];
             if (!isfinite(rznew)) flags |= kSolveNonFinite;
             if (MP && (mg || single))
-                beta = (rznew - get_total(P, RED_RZO, s_red)) / rz;  // Polak-Ribiere
+                beta = (rznew - s_total[1]) / rz;  // Polak-Ribiere
             else
                 beta = rznew / rz;
             rz = rznew;
         }
+        init = false;
+        if (it >= sP.maxit) {
+            ok = true;
+            break;
+        }
     }
 
-    // zero-mean projection of psi
-    SYNC_OR(goto aborted);
-    {
+    if (ok && bb == 0.0) {
+        OWN_LOOP(c) sP.psi[c] = 0.f;
+    } else if (ok) {
+        // zero-mean projection of psi (each thread's own cells, which no other thread has written)
+        const float *area = sP.area;
+        float *psi = sP.psi;
         double s = 0;
-        GRID_LOOP(c, n) s += (double)__ldg(P.area + c) * P.psi[c];
-        put_partial(P, RED_MEAN, s, s_red);
+#pragma unroll 4
+        OWN_LOOP(c) s += (double)__ldg(area + c) * psi[c];
+        ok = vsync(1, s, 0);
+        if (ok) {
+            const float m = (float)(s_total[0] / sP.total_area);
+#pragma unroll 4
+            OWN_LOOP(c) psi[c] -= m;
+            // leave the final residual / direction / preconditioned residual in the caller's buffers
+            if (r != sP.r) OWN_LOOP(c) sP.r[c] = r[c];
+            if (p != sP.p) OWN_LOOP(c) sP.p[c] = p[c];
+            if (z != sP.z) OWN_LOOP(c) sP.z[c] = z[c];
+        }
     }
-    SYNC_OR(goto aborted);
-    {
-        float m = (float)(get_total(P, RED_MEAN, s_red) / P.total_area);
-        GRID_LOOP(c, n) P.psi[c] -= m;
-        // leave the final residual / direction / preconditioned residual in the caller's buffers
-        if (r != P.r) GRID_LOOP(c, n) P.r[c] = r[c];
-        if (p != P.p) GRID_LOOP(c, n) P.p[c] = p[c];
-        if (z != P.z) GRID_LOOP(c, n) P.z[c] = z[c];
-    }
-    if (it >= P.maxit && rr > tol2) flags |= kSolveMaxit;
+done:
     if (vb() == 0 && threadIdx.x == 0) {
-        P.res->iters = it;
-        P.res->relres = sqrt(rr / bb);
-        P.res->status = 0;
-        P.res->r_final = 0;
-        P.res->flags = flags;
-        P.res->ns = globaltimer_ns() - t_begin;
-    }
-    return;
-
-aborted:
-    if (vb() == 0 && threadIdx.x == 0) {
-        P.res->iters = it;
-        P.res->relres = -1.0;
-        P.res->status = 1;
-        P.res->flags = flags | kSolveTimeout;
+        if (ok && it >= sP.maxit && rr > tol2) flags |= kSolveMaxit;
+        sP.res->iters = it;
+        sP.res->relres = !ok ? -1.0 : (bb == 0.0 ? 0.0 : sqrt(rr / bb));
+        sP.res->status = ok ? 0 : 1;
+        sP.res->r_final = 0;
+        sP.res->flags = ok ? flags : flags | kSolveTimeout;
+        if (ok) sP.res->ns = globaltimer_ns() - t_begin;
     }
 }
 
-// One solve on the whole grid, TPB threads per block.
+// One solve on the whole grid.
 template <bool MP, int TPB>
 __global__ void __launch_bounds__(TPB, 1) k_pcg(const __grid_constant__ SolveParams P) {
+    const int *src = reinterpret_cast<const int *>(&P);
+    int *dst = reinterpret_cast<int *>(&sP);
+    for (int k = threadIdx.x; k < (int)(sizeof(SolveParams) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
     if (threadIdx.x == 0) {
         s_vgrid[0] = blockIdx.x;
         s_vgrid[1] = gridDim.x;
+        s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP>(P);
+    pcg_body<MP>();
+}
+
+// Many planets' solves in one cooperative launch: block b runs planet
+// bmap[b].x's solve as block bmap[b].y of bmap[b].z (the planet's blocks are
+// consecutive), with that planet's parameters, barrier, partial sums and
+// result.  Planets finish independently.
+template <bool MP>
+__global__ void __launch_bounds__(kPB, 1) k_pcg_batch(const SolveParams *prm, const int4 *bmap) {
+    const int4 m = bmap[blockIdx.x];
+    const int *src = reinterpret_cast<const int *>(prm + m.x);
+    int *dst = reinterpret_cast<int *>(&sP);
+    for (int k = threadIdx.x; k < (int)(sizeof(SolveParams) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
+    if (threadIdx.x == 0) {
+        s_vgrid[0] = m.y;
+        s_vgrid[1] = m.z;
+        s_epoch = 0;
+    }
+    __syncthreads();
+    pcg_body<MP>();
 }
