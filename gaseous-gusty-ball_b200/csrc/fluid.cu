@@ -18,6 +18,7 @@ int pcg_max_blocks();
 int pcg_max_grid_n();
 void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks = 0);
 void levels_build(const SolveParams &P, LevelSet *out, std::vector<void *> &mem);
+void sweep_parts_build(const StencilDev &S, int blocks, SweepParts *out, std::vector<void *> &mem);
 void levels_build_mixed(const SolveParams &P, const LevelSet &plain, LevelSet *out, std::vector<void *> &mem);
 float *pcg_dense_map(const SolveParams &prm, int l0, int ld);
 
@@ -390,6 +391,7 @@ struct FluidPriv {
     LevelSet set[2] = {};           // what vcycle.cu builds for the plain and the mixed solve
     std::vector<void *> level_mem;  // its device arrays
     float *sw0 = nullptr, *sw1 = nullptr;  // sweeps of a coarsest level without a dense map
+    SweepParts sweep{};
     float *dense = nullptr;        // dense map of the V-cycle below the grid levels
     int nd = 0, ld = 0;
     int last_flags = 0;            // kSolve* bits of the last solve
@@ -527,6 +529,7 @@ static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int ma
     }
     P.sw0 = Pv->sw0;
     P.sw1 = Pv->sw1;
+    P.sweep = Pv->sweep;
     if (mg && Pv->dense) {
         P.dense = Pv->dense;
         P.nd = Pv->nd;
@@ -546,6 +549,7 @@ static void finish_levels(Fluid *F, FluidPriv *Pv) {
         const size_t n = P.L[Pv->nlev - 1].S.n;
         Pv->sw0 = (float *)dev_alloc(sizeof(float) * n);
         Pv->sw1 = (float *)dev_alloc(sizeof(float) * n);
+        if (P.coarse_on_grid) sweep_parts_build(P.L[Pv->nlev - 1].S, pcg_max_blocks(), &Pv->sweep, Pv->level_mem);
     }
 }
 

@@ -37,6 +37,21 @@ struct LevelDev {
     const int *ring_cell;   // [6 nring] ring cell | its on-face lanes << 24
 };
 
+// A coarsest level without a dense map, cut into parts (one per block) that
+// sweep by themselves for `depth` sweeps between exchanges: each part holds its
+// own cells and all cells within depth links of them, ordered by that distance.
+// count[p][h]: cells of part p within h links; the rest is indexed [p][slot] or
+// [p][link][slot] with kSweepSlots slots a part.
+constexpr int kSweepSlots = 1024;
+constexpr int kSweepDepth = 24;
+struct SweepParts {
+    int parts, depth;
+    const int *count;          // [parts][kSweepDepth + 1]
+    const int *cell;           // [parts][kSweepSlots]
+    const unsigned short *nb;  // [parts][8][kSweepSlots] slots of the neighbours (of cells within depth - 1 links)
+    const float *w;            // [parts][8][kSweepSlots]
+};
+
 // What levels_build (vcycle.cu) makes of a hierarchy, per precision.
 struct LevelSet {
     const float *rw16[kMaxLev];
@@ -87,6 +102,7 @@ struct SolveParams {
     SolveResult *res;
     // dense form of the V-cycle below the grid levels: xo_G = D b_G
     float *sw0, *sw1;    // the coarsest level's sweeps (coarse_on_grid)
+    SweepParts sweep;    // (parts = 0: the level is too large)
     const float *dense;  // [nd][ld] row-major (rows padded with zeros to ld), or nullptr
     int nd, ld;          // cells of level nlev_grid; row stride, a multiple of 4
 };

@@ -80,9 +80,18 @@ int pcg_max_blocks() { return device_sm_count(); }
 // bound is the one fluid_init's callers have always had).
 int pcg_max_grid_n() { return 1535; }
 
-static const void *pcg_kernel(bool mixed, int threads) {
-    if (threads == kPBWide) return mixed ? (const void *)k_pcg<true, kPBWide> : (const void *)k_pcg<false, kPBWide>;
-    return mixed ? (const void *)k_pcg<true, kPB> : (const void *)k_pcg<false, kPB>;
+template <bool MP>
+static const void *pcg_kernel(int threads, bool sweeps) {
+    if (threads == kPBWide)
+        return sweeps ? (const void *)k_pcg<MP, kPBWide, true> : (const void *)k_pcg<MP, kPBWide, false>;
+    return sweeps ? (const void *)k_pcg<MP, kPB, true> : (const void *)k_pcg<MP, kPB, false>;
+}
+static const void *pcg_kernel(bool mixed, int threads, bool sweeps) {
+    return mixed ? pcg_kernel<true>(threads, sweeps) : pcg_kernel<false>(threads, sweeps);
+}
+static const void *batch_kernel(bool mixed, bool sweeps) {
+    if (mixed) return sweeps ? (const void *)k_pcg_batch<true, true> : (const void *)k_pcg_batch<true, false>;
+    return sweeps ? (const void *)k_pcg_batch<false, true> : (const void *)k_pcg_batch<false, false>;
 }
 
 // Threads per block of a single solve on a grid of edge N.
@@ -91,11 +100,12 @@ static int pcg_threads(int N) { return N >= kWideMinN ? kPBWide : kPB; }
 static void pcg_attributes() {
     static bool attr = false;
     if (!attr) {
-        const void *ks[] = {pcg_kernel(false, kPB),     pcg_kernel(true, kPB),
-                            pcg_kernel(false, kPBWide), pcg_kernel(true, kPBWide),
-                            (const void *)k_pcg_batch<false>, (const void *)k_pcg_batch<true>};
-        for (const void *k : ks)
-            GGB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
+        for (int m = 0; m < 8; m++)
+            GGB_CHECK(cudaFuncSetAttribute(pcg_kernel(m & 1, m & 2 ? kPBWide : kPB, m & 4),
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
+        for (int m = 0; m < 4; m++)
+            GGB_CHECK(cudaFuncSetAttribute(batch_kernel(m & 1, m & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kStageBytes));
         GGB_CHECK(cudaFuncSetAttribute(k_dense_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr = true;
     }
@@ -114,7 +124,7 @@ void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks) {
     SolveParams p = prm;
     void *args[] = {&p};
     const int threads = pcg_threads(p.L[0].S.N);
-    const void *kernel = pcg_kernel(p.mixed != 0, threads);
+    const void *kernel = pcg_kernel(p.mixed != 0, threads, p.coarse_on_grid != 0);
     int grid = blocks_resident(kernel, threads);
     if (max_blocks > 0) grid = std::max(1, std::min(grid, max_blocks));
     GGB_CHECK(cudaMemsetAsync(&p.bar->count, 0, sizeof(unsigned int), s));
@@ -125,14 +135,16 @@ void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks) {
 // Blocks of one batched solve launch that can be resident at once (the
 // launch's capacity).
 int pcg_batch_capacity(bool mixed) {
-    return blocks_resident(mixed ? (const void *)k_pcg_batch<true> : (const void *)k_pcg_batch<false>, kPB);
+    return blocks_resident(batch_kernel(mixed, true), kPB);
 }
 
 // One cooperative launch of nblocks blocks solving every planet of a batch
 // (dev_prm: the planets' parameters; dev_bmap: block -> planet, block of the
-// planet, blocks of the planet).  The planets' barrier counters must be zero.
-void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, bool mixed, cudaStream_t s) {
-    const void *k = mixed ? (const void *)k_pcg_batch<true> : (const void *)k_pcg_batch<false>;
+// planet, blocks of the planet; sweeps: some planet has no dense map).  The
+// planets' barrier counters must be zero.
+void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, bool mixed, bool sweeps,
+                      cudaStream_t s) {
+    const void *k = batch_kernel(mixed, sweeps);
     void *args[] = {(void *)&dev_prm, (void *)&dev_bmap};
     GGB_CHECK(cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(kPB), args, kStageBytes, s));
     GGB_LAUNCHED();

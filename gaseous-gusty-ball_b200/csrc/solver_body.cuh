@@ -27,6 +27,7 @@ constexpr double kCorrScale = 1.0;  // upstream MG_CORR_SCALE
 // region).
 constexpr int kMaxN = 1535;
 constexpr int kWinCap = (kChunk + 2 * kMaxN + 2 + 3) & ~3;  // whole 16-byte groups: the pool follows
+static_assert(kWinCap >= 2 * kSweepSlots, "two buffers of a part's values");
 static_assert(kWinCap >= 3 * kBlockSweepMax, "x, xo and b of a level that one block sweeps");
 constexpr int kSlotPool = 34816;
 static_assert(kSlotPool >= 4 * (kChunk + 2 * kMaxN + 2 + 8), "a chunk's slot weights fit");
@@ -654,15 +655,101 @@ __device__ __forceinline__ void dense_rows(const DenseTaps &T, Get4 get4, Put pu
     }
 }
 
-// The coarsest level's damped-Jacobi sweeps from 0, grid-wide, in FP32
-// (upstream src/fluid.c:118-137), for a level too large for the dense map.
-// With a thread for every cell its links stay in registers, so that a sweep is
-// one gather round and one grid barrier.  Returns the buffer that holds the
-// result (read at the own cell only), or nullptr on abort.
-template <bool MP, class GetB>
-__device__ __forceinline__ const float *coarse_sweeps(const LevelDev &L, GetB getb) {
-    const int n = L.S.n;
+// The coarsest level's damped-Jacobi sweeps from 0 (upstream src/fluid.c:118-137)
+// for a level without a dense map: FP32, each sweep rounded to the storage type;
+// put(c, x) with the result.  False on abort.  (Only in the kernels' SWEEPS
+// variants: in the same kernel as the dense map, inlined or as a call, its
+// registers cost the solve at N = 256 9 to 12 %.)
+//
+// A level cut into parts (SweepParts) sweeps `depth` times between exchanges, in
+// shared memory with the links in registers: after an exchange a part holds every
+// cell within depth links of its own, and each sweep is valid one link less far
+// out, so cells near a part's edge are swept by several blocks, to the same
+// values.  60 sweeps of 3750 cells (N = 100: 25) then take 7 grid barriers instead
+// of 60, and the coarsest level 38 us a V-cycle instead of 250.  A larger level,
+// or a solve on fewer blocks than parts, sweeps grid-wide with a barrier per
+// sweep; with a thread for every cell its links stay in registers there too.
+template <bool MP, class GetB, class Put>
+__device__ __forceinline__ bool coarse_sweeps(const LevelDev &L, GetB getb, Put put) {
+    const int n = L.S.n, sweeps = sP.coarse_sweeps;
     float *src = sP.sw0, *dst = sP.sw1;
+    if (sP.sweep.parts > 0 && vnb() >= sP.sweep.parts) {
+        constexpr int kPer = 2;  // slots per thread (kSweepSlots / 512)
+        const SweepParts &W = sP.sweep;
+        const int part = vb(), depth = W.depth, bs = blockDim.x;
+        const bool mine = part < W.parts;
+        const int *cnt = W.count + (size_t)(mine ? part : 0) * (kSweepDepth + 1);
+        const int own = mine ? __ldg(cnt) : 0, all = mine ? __ldg(cnt + depth) : 0;
+        float *xs = s_win(), *xd = xs + kSweepSlots;
+        int cell[kPer];
+        unsigned nb[kPer][kMaxNb / 2];
+        float wv[kPer][kMaxNb], bc[kPer];
+        double od[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const int s = threadIdx.x + u * bs;
+            if (s >= all) continue;
+            cell[u] = __ldg(W.cell + (size_t)part * kSweepSlots + s);
+#pragma unroll
+            for (int k = 0; k < kMaxNb; k++) {
+                const size_t at = ((size_t)part * kMaxNb + k) * kSweepSlots + s;
+                const unsigned o = __ldg(W.nb + at);
+                nb[u][k / 2] = k & 1 ? nb[u][k / 2] | o << 16 : o;
+                wv[u][k] = __ldg(W.w + at);
+            }
+            bc[u] = getb(cell[u]);
+            od[u] = kOmegaJ * __ldg(L.dinv + cell[u]);
+            xs[s] = as_stored<MP>((float)(od[u] * bc[u]));  // the first sweep
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int done = 1;;) {
+            const int run = min(depth, sweeps - done);
+#pragma unroll 1
+            for (int left = run - 1; left >= 0; left--) {
+                const int lim = mine ? __ldg(cnt + left) : 0;
+#pragma unroll
+                for (int u = 0; u < kPer; u++) {
+                    const int s = threadIdx.x + u * bs;
+                    if (s >= lim) continue;
+                    const float xc = xs[s];
+                    double acc = 0;
+#pragma unroll
+                    for (int k = 0; k < kMaxNb; k++)
+                        acc += (double)wv[u][k] *
+                               ((double)xc - (double)xs[k & 1 ? nb[u][k / 2] >> 16 : nb[u][k / 2] & 0xffffu]);
+                    const float rc = (float)(bc[u] - acc);
+                    xd[s] = as_stored<MP>(xc + (float)(od[u] * rc));
+                }
+                __syncthreads();
+                float *t = xs;
+                xs = xd;
+                xd = t;
+            }
+            done += run;
+            if (done >= sweeps) break;
+            // own values out, those around the part in
+#pragma unroll
+            for (int u = 0; u < kPer; u++)
+                if ((int)threadIdx.x + u * bs < own) dst[cell[u]] = xs[threadIdx.x + u * bs];
+            if (!vsync(0, 0, 0)) return false;
+            const int need = mine ? __ldg(cnt + min(depth, sweeps - done)) : 0;
+#pragma unroll
+            for (int u = 0; u < kPer; u++) {
+                const int s = threadIdx.x + u * bs;
+                if (s >= own && s < need) xs[s] = dst[cell[u]];
+            }
+            __syncthreads();
+            float *t = src;
+            src = dst;
+            dst = t;
+        }
+#pragma unroll
+        for (int u = 0; u < kPer; u++)
+            if ((int)threadIdx.x + u * bs < own) put(cell[u], xs[threadIdx.x + u * bs]);
+        __syncthreads();
+        return true;
+    }
     if (n <= vnb() * (int)blockDim.x) {
         const int c = vb() * blockDim.x + threadIdx.x;
         int nb[kMaxNb];
@@ -676,8 +763,8 @@ __device__ __forceinline__ const float *coarse_sweeps(const LevelDev &L, GetB ge
             src[c] = xc;
         }
 #pragma unroll 1
-        for (int s = 1; s < sP.coarse_sweeps; s++) {
-            if (!vsync(0, 0, 0)) return nullptr;
+        for (int s = 1; s < sweeps; s++) {
+            if (!vsync(0, 0, 0)) return false;
             if (c < n) {
                 float v[kMaxNb];
 #pragma unroll
@@ -693,17 +780,20 @@ __device__ __forceinline__ const float *coarse_sweeps(const LevelDev &L, GetB ge
             src = dst;
             dst = t;
         }
-        return src;
+        if (c < n) put(c, xc);
+        return true;
     }
     GRID_LOOP(c, n) src[c] = as_stored<MP>((float)(kOmegaJ * __ldg(L.dinv + c) * getb(c)));
-    for (int s = 1; s < sP.coarse_sweeps; s++) {
-        if (!vsync(0, 0, 0)) return nullptr;
+#pragma unroll 1
+    for (int s = 1; s < sweeps; s++) {
+        if (!vsync(0, 0, 0)) return false;
         GRID_LOOP(c, n) dst[c] = as_stored<MP>(jacobi_cell(L.S, L.dinv, getb(c), src, c));
         float *t = src;
         src = dst;
         dst = t;
     }
-    return src;
+    GRID_LOOP(c, n) put(c, src[c]);
+    return true;
 }
 
 // ---- the grid levels of the V-cycle ------------------------------------------
@@ -811,7 +901,8 @@ __device__ __forceinline__ float vscale(double rr, int n) {
 }
 
 // The whole solve of this block's planet (sP) on the block's virtual grid.
-template <bool MP>
+// SWEEPS: with the sweeps of a coarsest level that has no dense map.
+template <bool MP, bool SWEEPS>
 __device__ __forceinline__ void pcg_body() {
     using A = typename Prec<MP>::A;
     using V = typename Prec<MP>::V;
@@ -1049,10 +1140,8 @@ __device__ __forceinline__ void pcg_body() {
                         coarsest_smem(L, lvl, sP.coarse_sweeps);
                         BLOCK_LOOP(c, n) put(c, MP ? lvl.xo[c] * s0 : lvl.xo[c]);
                     }
-                } else {
-                    const float *x = coarse_sweeps<MP>(L, getb);
-                    if (!x) goto done;
-                    GRID_LOOP(c, L.S.n) put(c, x[c]);
+                } else if (SWEEPS) {
+                    if (!coarse_sweeps<MP>(L, getb, put)) goto done;
                 }
             }
             if (mg) {
@@ -1139,7 +1228,7 @@ done:
 }
 
 // One solve on the whole grid.
-template <bool MP, int TPB>
+template <bool MP, int TPB, bool SWEEPS>
 __global__ void __launch_bounds__(TPB, 1) k_pcg(const __grid_constant__ SolveParams P) {
     const int *src = reinterpret_cast<const int *>(&P);
     int *dst = reinterpret_cast<int *>(&sP);
@@ -1150,14 +1239,14 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg(const __grid_constant__ SolvePar
         s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP>();
+    pcg_body<MP, SWEEPS>();
 }
 
 // Many planets' solves in one cooperative launch: block b runs planet
 // bmap[b].x's solve as block bmap[b].y of bmap[b].z (the planet's blocks are
 // consecutive), with that planet's parameters, barrier, partial sums and
 // result.  Planets finish independently.
-template <bool MP>
+template <bool MP, bool SWEEPS>
 __global__ void __launch_bounds__(kPB, 1) k_pcg_batch(const SolveParams *prm, const int4 *bmap) {
     const int4 m = bmap[blockIdx.x];
     const int *src = reinterpret_cast<const int *>(prm + m.x);
@@ -1169,5 +1258,5 @@ __global__ void __launch_bounds__(kPB, 1) k_pcg_batch(const SolveParams *prm, co
         s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP>();
+    pcg_body<MP, SWEEPS>();
 }

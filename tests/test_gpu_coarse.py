@@ -24,7 +24,7 @@ def rel_l2(a, b):
 
 
 @pytest.mark.parametrize("N,mixed", [(4, 0), (5, 1), (27, 0), (31, 1), (33, 0), (33, 1), (50, 0), (50, 1), (62, 0),
-                                     (66, 0), (66, 1), (100, 0)])
+                                     (66, 0), (66, 1), (100, 0), (45, 0), (90, 1), (150, 0), (198, 0)])
 def test_poisson_coarse_forms(gpu, orc64, N, mixed):
     ref = K.poisson(orc64, N, tol=1e-10, tables=K.tables_of(gpu, N))
     got = K.poisson(gpu, N, tol=1e-6, mixed=bool(mixed))
