@@ -104,8 +104,9 @@ int fluid_solve_mixed(const Fluid *F);
 double fluid_last_solve_seconds(const Fluid *F);
 void fluid_result_velocity_queue(Fluid *F);
 int pcg_batch_capacity(bool mixed);
-void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, bool mixed, bool sweeps,
-                      cudaStream_t s);
+void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, int threads, bool mixed,
+                      bool sweeps, cudaStream_t s);
+int pcg_batch_threads(long long cells, int nblocks, int alone_n);
 void render_deposit_queue(Render *r, const Particles *P);
 void render_deposit_collect(Render *r, const Particles *P);
 void particles_advect_queue(Particles *P, const CubeSphere *cs, const float *vel, const double *dt_dev);

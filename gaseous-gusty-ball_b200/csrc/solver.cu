@@ -89,13 +89,29 @@ static const void *pcg_kernel(int threads, bool sweeps) {
 static const void *pcg_kernel(bool mixed, int threads, bool sweeps) {
     return mixed ? pcg_kernel<true>(threads, sweeps) : pcg_kernel<false>(threads, sweeps);
 }
-static const void *batch_kernel(bool mixed, bool sweeps) {
-    if (mixed) return sweeps ? (const void *)k_pcg_batch<true, true> : (const void *)k_pcg_batch<true, false>;
-    return sweeps ? (const void *)k_pcg_batch<false, true> : (const void *)k_pcg_batch<false, false>;
+template <bool MP>
+static const void *batch_kernel(int threads, bool sweeps) {
+    if (threads == kPBWide)
+        return sweeps ? (const void *)k_pcg_batch<MP, kPBWide, true> : (const void *)k_pcg_batch<MP, kPBWide, false>;
+    return sweeps ? (const void *)k_pcg_batch<MP, kPB, true> : (const void *)k_pcg_batch<MP, kPB, false>;
+}
+static const void *batch_kernel(bool mixed, int threads, bool sweeps) {
+    return mixed ? batch_kernel<true>(threads, sweeps) : batch_kernel<false>(threads, sweeps);
 }
 
 // Threads per block of a single solve on a grid of edge N.
 static int pcg_threads(int N) { return N >= kWideMinN ? kPBWide : kPB; }
+
+// ... of a batched launch over nblocks blocks for grids of `cells` cells in all:
+// with many cells per block the chunks' loads bound a phase, not its barrier, and
+// twice the warps keep twice as many in flight (12 planets of 64 to 256 cells an
+// edge, 8600 cells per block, mixed: 2.47 ms with 512 threads, 1.76 with 1024; 4
+// planets, 3650: 1.02 and 1.05; 2 planets, 830: 0.50 and 0.61).  alone: one planet
+// on the whole launch, with fluid_step's choice (and so its sums).
+int pcg_batch_threads(long long cells, int nblocks, int alone_n) {
+    if (alone_n > 0) return pcg_threads(alone_n);
+    return cells > (long long)kWideBatchCells * nblocks ? kPBWide : kPB;
+}
 
 static void pcg_attributes() {
     static bool attr = false;
@@ -103,9 +119,9 @@ static void pcg_attributes() {
         for (int m = 0; m < 8; m++)
             GGB_CHECK(cudaFuncSetAttribute(pcg_kernel(m & 1, m & 2 ? kPBWide : kPB, m & 4),
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
-        for (int m = 0; m < 4; m++)
-            GGB_CHECK(cudaFuncSetAttribute(batch_kernel(m & 1, m & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)kStageBytes));
+        for (int m = 0; m < 8; m++)
+            GGB_CHECK(cudaFuncSetAttribute(batch_kernel(m & 1, m & 2 ? kPBWide : kPB, m & 4),
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
         GGB_CHECK(cudaFuncSetAttribute(k_dense_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr = true;
     }
@@ -135,18 +151,19 @@ void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks) {
 // Blocks of one batched solve launch that can be resident at once (the
 // launch's capacity).
 int pcg_batch_capacity(bool mixed) {
-    return blocks_resident(batch_kernel(mixed, true), kPB);
+    return std::min(blocks_resident(batch_kernel(mixed, kPB, true), kPB),
+                    blocks_resident(batch_kernel(mixed, kPBWide, true), kPBWide));
 }
 
 // One cooperative launch of nblocks blocks solving every planet of a batch
 // (dev_prm: the planets' parameters; dev_bmap: block -> planet, block of the
 // planet, blocks of the planet; sweeps: some planet has no dense map).  The
 // planets' barrier counters must be zero.
-void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, bool mixed, bool sweeps,
-                      cudaStream_t s) {
-    const void *k = batch_kernel(mixed, sweeps);
+void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, int threads, bool mixed,
+                      bool sweeps, cudaStream_t s) {
+    const void *k = batch_kernel(mixed, threads, sweeps);
     void *args[] = {(void *)&dev_prm, (void *)&dev_bmap};
-    GGB_CHECK(cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(kPB), args, kStageBytes, s));
+    GGB_CHECK(cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(threads), args, kStageBytes, s));
     GGB_LAUNCHED();
 }
 

@@ -18,6 +18,7 @@
 constexpr int kBlockSweepMax = 1536;  // cells of a level that one block sweeps in shared memory
 constexpr int kPB = 512;          // threads per block of the persistent kernel
 constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh the phases' latency
+constexpr int kWideBatchCells = 4000;  // mean cells per block of a batched launch from which its blocks are wide
 constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 256 0.756 / 0.906, 448 1.57 / 1.68, 512 1.97 / 1.92
 constexpr int kChunk = 3072;      // cells of a stencil chunk
 constexpr double kOmegaJ = 0.8;      // upstream MG_OMEGA
@@ -1246,8 +1247,8 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg(const __grid_constant__ SolvePar
 // bmap[b].x's solve as block bmap[b].y of bmap[b].z (the planet's blocks are
 // consecutive), with that planet's parameters, barrier, partial sums and
 // result.  Planets finish independently.
-template <bool MP, bool SWEEPS>
-__global__ void __launch_bounds__(kPB, 1) k_pcg_batch(const SolveParams *prm, const int4 *bmap) {
+template <bool MP, int TPB, bool SWEEPS>
+__global__ void __launch_bounds__(TPB, 1) k_pcg_batch(const SolveParams *prm, const int4 *bmap) {
     const int4 m = bmap[blockIdx.x];
     const int *src = reinterpret_cast<const int *>(prm + m.x);
     int *dst = reinterpret_cast<int *>(&sP);
