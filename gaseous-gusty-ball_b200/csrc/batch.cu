@@ -169,7 +169,7 @@ static void plan(GGBBatch *b) {
     int total = 0;
     for (int m = 0; m < 2; m++) {
         if (order[m].empty()) continue;
-        const int cap = pcg_batch_capacity(m == 1);
+        const int cap = pcg_batch_capacity();
         if (b->fixed_blocks >= cap) {
             // every planet alone on the whole launch: one launch per planet,
             // the same blocks (and so the same arithmetic) as fluid_step's solve
@@ -334,7 +334,7 @@ GGB_EXPORT int ggb_batch_step(GGBBatch *b, int steps) {
                 sweeps |= b->prm_host[i].coarse_on_grid != 0;
             }
             const bool mixed = fluid_solve_mixed(b->F[grp[0]]) != 0;
-            const int alone = grp.size() == 1 && nb >= pcg_batch_capacity(mixed) ? grid_n(b, grp[0]) : 0;
+            const int alone = grp.size() == 1 && nb >= pcg_batch_capacity() ? grid_n(b, grp[0]) : 0;
             pcg_launch_batch(b->prm_dev, b->bmap_dev + q, nb, pcg_batch_threads(cells, nb, alone), mixed, sweeps, base);
             q += nb;
         }

@@ -103,7 +103,7 @@ void fluid_step_solve_params(Fluid *F, GridBarrier *bar, SolveParams *out);
 int fluid_solve_mixed(const Fluid *F);
 double fluid_last_solve_seconds(const Fluid *F);
 void fluid_result_velocity_queue(Fluid *F);
-int pcg_batch_capacity(bool mixed);
+int pcg_batch_capacity();
 void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, int threads, bool mixed,
                       bool sweeps, cudaStream_t s);
 int pcg_batch_threads(long long cells, int nblocks, int alone_n);

@@ -35,6 +35,7 @@
 //     blocks from L2.
 #include <algorithm>
 #include <cstdio>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -84,6 +85,8 @@ template <bool MP>
 static const void *pcg_kernel(int threads, bool sweeps) {
     if (threads == kPBWide)
         return sweeps ? (const void *)k_pcg<MP, kPBWide, true> : (const void *)k_pcg<MP, kPBWide, false>;
+    if (threads == kPBNarrow)
+        return sweeps ? (const void *)k_pcg<MP, kPBNarrow, true> : (const void *)k_pcg<MP, kPBNarrow, false>;
     return sweeps ? (const void *)k_pcg<MP, kPB, true> : (const void *)k_pcg<MP, kPB, false>;
 }
 static const void *pcg_kernel(bool mixed, int threads, bool sweeps) {
@@ -93,6 +96,8 @@ template <bool MP>
 static const void *batch_kernel(int threads, bool sweeps) {
     if (threads == kPBWide)
         return sweeps ? (const void *)k_pcg_batch<MP, kPBWide, true> : (const void *)k_pcg_batch<MP, kPBWide, false>;
+    if (threads == kPBNarrow)
+        return sweeps ? (const void *)k_pcg_batch<MP, kPBNarrow, true> : (const void *)k_pcg_batch<MP, kPBNarrow, false>;
     return sweeps ? (const void *)k_pcg_batch<MP, kPB, true> : (const void *)k_pcg_batch<MP, kPB, false>;
 }
 static const void *batch_kernel(bool mixed, int threads, bool sweeps) {
@@ -100,7 +105,10 @@ static const void *batch_kernel(bool mixed, int threads, bool sweeps) {
 }
 
 // Threads per block of a single solve on a grid of edge N.
-static int pcg_threads(int N) { return N >= kWideMinN ? kPBWide : kPB; }
+static int pcg_threads(int N) {
+    if (N >= kWideMinN) return kPBWide;
+    return 6LL * N * N <= (long long)kNarrowCells * device_sm_count() ? kPBNarrow : kPB;
+}
 
 // ... of a batched launch over nblocks blocks for grids of `cells` cells in all:
 // with many cells per block the chunks' loads bound a phase, not its barrier, and
@@ -110,28 +118,24 @@ static int pcg_threads(int N) { return N >= kWideMinN ? kPBWide : kPB; }
 // on the whole launch, with fluid_step's choice (and so its sums).
 int pcg_batch_threads(long long cells, int nblocks, int alone_n) {
     if (alone_n > 0) return pcg_threads(alone_n);
-    return cells > (long long)kWideBatchCells * nblocks ? kPBWide : kPB;
+    if (cells > (long long)kWideBatchCells * nblocks) return kPBWide;
+    return cells <= (long long)kNarrowCells * nblocks ? kPBNarrow : kPB;
 }
 
-static void pcg_attributes() {
-    static bool attr = false;
-    if (!attr) {
-        for (int m = 0; m < 8; m++)
-            GGB_CHECK(cudaFuncSetAttribute(pcg_kernel(m & 1, m & 2 ? kPBWide : kPB, m & 4),
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
-        for (int m = 0; m < 8; m++)
-            GGB_CHECK(cudaFuncSetAttribute(batch_kernel(m & 1, m & 2 ? kPBWide : kPB, m & 4),
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
-        GGB_CHECK(cudaFuncSetAttribute(k_dense_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr = true;
-    }
-}
-
+// Blocks of a launch of `kernel`.  A variant is looked at (and with lazy loading
+// brought to the device) when it is first launched: all 24 at once cost a program's
+// first solve 40 ms.
 static int blocks_resident(const void *kernel, int threads) {
-    pcg_attributes();
-    int per = 0;
-    GGB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, kStageBytes));
-    if (per < 1) fail_msg("the solve kernel cannot be resident on this device (%zu B shared memory)", kStageBytes);
+    static std::mutex m;
+    static std::vector<const void *> ready;
+    std::lock_guard<std::mutex> lock(m);
+    if (std::find(ready.begin(), ready.end(), kernel) == ready.end()) {
+        GGB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes));
+        int per = 0;
+        GGB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, kStageBytes));
+        if (per < 1) fail_msg("the solve kernel cannot be resident on this device (%zu B shared memory)", kStageBytes);
+        ready.push_back(kernel);
+    }
     return device_sm_count();  // one block per SM: more would only add arrivals to every barrier
 }
 
@@ -150,10 +154,7 @@ void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks) {
 
 // Blocks of one batched solve launch that can be resident at once (the
 // launch's capacity).
-int pcg_batch_capacity(bool mixed) {
-    return std::min(blocks_resident(batch_kernel(mixed, kPB, true), kPB),
-                    blocks_resident(batch_kernel(mixed, kPBWide, true), kPBWide));
-}
+int pcg_batch_capacity() { return device_sm_count(); }
 
 // One cooperative launch of nblocks blocks solving every planet of a batch
 // (dev_prm: the planets' parameters; dev_bmap: block -> planet, block of the
@@ -162,6 +163,7 @@ int pcg_batch_capacity(bool mixed) {
 void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, int threads, bool mixed,
                       bool sweeps, cudaStream_t s) {
     const void *k = batch_kernel(mixed, threads, sweeps);
+    blocks_resident(k, threads);
     void *args[] = {(void *)&dev_prm, (void *)&dev_bmap};
     GGB_CHECK(cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(threads), args, kStageBytes, s));
     GGB_LAUNCHED();
@@ -175,7 +177,7 @@ float *pcg_dense_map(const SolveParams &prm, int l0, int ld) {
     size_t cells = 0;
     for (int l = l0; l < p.nlev; l++) cells += p.L[l].S.n;
     size_t smem = 4 * sizeof(float) * cells;
-    pcg_attributes();
+    GGB_CHECK(cudaFuncSetAttribute(k_dense_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     int grid = std::min(nd, 4 * device_sm_count());
     k_dense_columns<<<grid, kPB, smem, stream()>>>(p, l0, D, ld);
     GGB_LAUNCHED();

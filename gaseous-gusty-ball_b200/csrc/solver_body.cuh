@@ -16,8 +16,16 @@
 // 0.775 and 2.23, 1.93.  The FP32 and FP16 roundings of every vector are unchanged.
 
 constexpr int kBlockSweepMax = 1536;  // cells of a level that one block sweeps in shared memory
-constexpr int kPB = 512;          // threads per block of the persistent kernel
+constexpr int kPBNarrow = 384;   // threads per block of the persistent kernel on small grids
+constexpr int kPB = 512;         // ... on ordinary ones
 constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh the phases' latency
+// Cells per block up to which blocks are narrow: with few cells a thread, a
+// phase's time is its barrier and the issue of the warps' common part (sums,
+// index arithmetic, block barriers), of which 12 warps have less than 16.  512 /
+// 384 threads on 148 SMs, ms: N = 32 0.178 / 0.169, 64 0.241 / 0.230, 128 0.495 /
+// 0.477, 192 0.626 / 0.622, 256 (2657 cells) 0.759 / 0.758, 384 1.25 / 1.34; 256
+// and 320 threads are slower from N = 128 on (0.522, 0.504).
+constexpr int kNarrowCells = 2700;
 constexpr int kWideBatchCells = 4000;  // mean cells per block of a batched launch from which its blocks are wide
 constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 256 0.756 / 0.906, 448 1.57 / 1.68, 512 1.97 / 1.92
 constexpr int kChunk = 3072;      // cells of a stencil chunk
@@ -670,12 +678,12 @@ __device__ __forceinline__ void dense_rows(const DenseTaps &T, Get4 get4, Put pu
 // of 60, and the coarsest level 38 us a V-cycle instead of 250.  A larger level,
 // or a solve on fewer blocks than parts, sweeps grid-wide with a barrier per
 // sweep; with a thread for every cell its links stay in registers there too.
-template <bool MP, class GetB, class Put>
+template <bool MP, int TPB, class GetB, class Put>
 __device__ __forceinline__ bool coarse_sweeps(const LevelDev &L, GetB getb, Put put) {
     const int n = L.S.n, sweeps = sP.coarse_sweeps;
     float *src = sP.sw0, *dst = sP.sw1;
     if (sP.sweep.parts > 0 && vnb() >= sP.sweep.parts) {
-        constexpr int kPer = 2;  // slots per thread (kSweepSlots / 512)
+        constexpr int kPer = (kSweepSlots + TPB - 1) / TPB;  // slots per thread
         const SweepParts &W = sP.sweep;
         const int part = vb(), depth = W.depth, bs = blockDim.x;
         const bool mine = part < W.parts;
@@ -903,7 +911,7 @@ __device__ __forceinline__ float vscale(double rr, int n) {
 
 // The whole solve of this block's planet (sP) on the block's virtual grid.
 // SWEEPS: with the sweeps of a coarsest level that has no dense map.
-template <bool MP, bool SWEEPS>
+template <bool MP, int TPB, bool SWEEPS>
 __device__ __forceinline__ void pcg_body() {
     using A = typename Prec<MP>::A;
     using V = typename Prec<MP>::V;
@@ -1142,7 +1150,7 @@ __device__ __forceinline__ void pcg_body() {
                         BLOCK_LOOP(c, n) put(c, MP ? lvl.xo[c] * s0 : lvl.xo[c]);
                     }
                 } else if (SWEEPS) {
-                    if (!coarse_sweeps<MP>(L, getb, put)) goto done;
+                    if (!coarse_sweeps<MP, TPB>(L, getb, put)) goto done;
                 }
             }
             if (mg) {
@@ -1240,7 +1248,7 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg(const __grid_constant__ SolvePar
         s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP, SWEEPS>();
+    pcg_body<MP, TPB, SWEEPS>();
 }
 
 // Many planets' solves in one cooperative launch: block b runs planet
@@ -1259,5 +1267,5 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg_batch(const SolveParams *prm, co
         s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP, SWEEPS>();
+    pcg_body<MP, TPB, SWEEPS>();
 }

@@ -69,3 +69,14 @@ def test_batched_solve_on_few_blocks(gpu, orc64, N, mixed, blocks):
     assert relres <= 1e-6
     assert rel_l2(got["psi"], ref["psi"]) <= 1e-5
     assert rel_l2(got["vel"], ref["vel"]) <= 5e-5
+
+
+@pytest.mark.parametrize("N,mixed", [(256, 1), (258, 0), (258, 1), (260, 0), (262, 1)])
+def test_poisson_narrow_block_sizes(gpu, orc64, N, mixed):
+    """Both sides of the mean cells per block up to which blocks have 384
+    threads; bounds as above."""
+    ref = K.poisson(orc64, N, tol=1e-10, tables=K.tables_of(gpu, N))
+    got = K.poisson(gpu, N, tol=1e-6, mixed=bool(mixed))
+    assert float(got["relres"]) <= 1e-6
+    assert rel_l2(got["psi"], ref["psi"]) <= 1e-5
+    assert rel_l2(got["vel"], ref["vel"]) <= 5e-5
