@@ -197,26 +197,14 @@ __device__ __forceinline__ bool vsync(int nv, double v0, double v1, bool late = 
     return s_ok != 0;
 }
 
-// This block's contiguous range of a level's n = 6 N^2 cells (face-major).
-// With at least 6 blocks every face gets a whole number of blocks (face f:
-// blocks [f nb / 6, (f + 1) nb / 6)) and splits its cells evenly among them,
-// so that no range holds the boundary rows of two faces: a range straddling a
-// face edge has twice the boundary-ring cells, which takes a second link pass
-// (or, at N = 512, another sub-range) and makes that block the phase's last.
-// Fewer blocks split the cells evenly.
-__device__ __forceinline__ void block_range(int n, int N, int &c0, int &c1) {
-    const int nb = vnb(), b = vb();
-    if (nb < 6) {
-        c0 = (int)(((long long)n * b) / nb);
-        c1 = (int)(((long long)n * (b + 1)) / nb);
-        return;
-    }
-    int f = 0;
-    while (f < 5 && b >= ((f + 1) * nb) / 6) f++;
-    const int b0 = (f * nb) / 6, m = ((f + 1) * nb) / 6 - b0;
-    const long long nf = (long long)N * N;
-    c0 = (int)(f * nf + nf * (b - b0) / m);
-    c1 = (int)(f * nf + nf * (b - b0 + 1) / m);
+// This block's contiguous range of a level's n cells (face-major), the same
+// number for every block whatever faces they lie on: the boundary-ring cells are
+// dealt over the grid apart from the ranges.  (With whole blocks per face a solve
+// on 11 blocks took as long as on 6: 10 planets of 64 to 256 cells an edge, whose
+// shares move by a block from run to run, 1.71 to 2.27 ms; this way 1.63 to 1.73.)
+__device__ __forceinline__ void block_range(int n, int &c0, int &c1) {
+    c0 = (int)(((long long)n * vb()) / vnb());
+    c1 = (int)(((long long)n * (vb() + 1)) / vnb());
 }
 
 __device__ unsigned long long *g_stage_trace;  // diagnostics: block 0 stamps the stencil phases
@@ -273,7 +261,7 @@ __device__ __noinline__ void block_setup() {
         for (int l = 0; l < levels; l++) {
             const StencilDev &S = sP.L[l].S;
             int c0, c1;
-            block_range(S.n, S.N, c0, c1);
+            block_range(S.n, c0, c1);
             s_range[l][0] = c0;
             s_range[l][1] = c1;
             if (l >= slots) continue;

@@ -80,3 +80,26 @@ def test_poisson_narrow_block_sizes(gpu, orc64, N, mixed):
     assert float(got["relres"]) <= 1e-6
     assert rel_l2(got["psi"], ref["psi"]) <= 1e-5
     assert rel_l2(got["vel"], ref["vel"]) <= 5e-5
+
+
+@pytest.mark.parametrize("N,mixed", [(128, 0), (129, 1)])
+def test_block_count_does_not_change_the_solve(gpu, N, mixed):
+    """Shares of 5 to 12 blocks cut the cells anywhere on the faces: the same
+    psi from the same state, to 100 times the FP32 rounding (a sum in FP64 over
+    other partial sums moves an FP32 vector by an ulp now and then)."""
+    out = []
+    for blocks in (5, 6, 11, 12):
+        g = gpu.grid(N)
+        vel0, band = K.initial_velocity(gpu, g, seed=5)
+        fs = G.FluidSim(gpu, g, rotation=2.0, cg_tol=1e-6, mixed=bool(mixed))
+        fs.set_state(vel0, band)
+        F = (C.POINTER(gpu.T["Fluid"]) * 1)(C.pointer(fs.F))
+        b = gpu.lib.ggb_batch_create(1, F, None, None, (C.c_double * 1)(1.0), None)
+        gpu.lib.ggb_batch_solve_blocks(b, blocks)
+        assert gpu.lib.ggb_batch_step(b, 1) == 0
+        out.append(fs.field("psi").copy())
+        gpu.lib.ggb_batch_free(b)
+        fs.free()
+        g.free()
+    for psi in out[1:]:
+        assert rel_l2(psi, out[0]) <= 1.2e-5
