@@ -506,8 +506,12 @@ __global__ void __launch_bounds__(1024) k_tile_scan(int n, const unsigned *cnt, 
 // ---- tile compositing: one block per tile, one texel per thread ----------
 constexpr int kTB = kT * kT;   // threads per tile block: one texel each
 constexpr int kRec = 576;      // records of one window (shared memory)
-constexpr int kEnt = 1728;     // (record, texel) entries of one window
-constexpr int kHist = 1024;    // key buckets when a dense tile is cut into windows
+// (record, texel) entries of one window: as many as the one-pass slots' memory
+// holds.  At 1728, three a record, tiles of 450 records and more went in two
+// windows: splat stage N = 64 127 us, now 118; N = 256 402, now 394.
+constexpr int kEnt = 4608;
+constexpr int kHistBits = 10;
+constexpr int kHist = 1 << kHistBits;  // key buckets when a dense tile is cut into windows
 constexpr int kBucket = 16;    // entry slots per texel of the one-pass path
 constexpr int kBucketStride = 18;  // slots between texels: 9 words, so a warp's texels hit distinct banks
 
@@ -624,20 +628,36 @@ __device__ __forceinline__ void window_colours(TileSmem &S, int m, const float4 
     for (int s = threadIdx.x; s < m; s += blockDim.x) S.col[s] = __ldg(col + (S.u.r.key[s] >> 13));
 }
 
-// Blends the sorted entries e[0..m) of texel q into d (upstream
-// src/render.c:135-151).
-__device__ __forceinline__ void blend_texel(const TileSmem &S, unsigned short *e, int m, int q, const SplatCfg &C,
-                                            const TileGeo &G, float4 &d) {
-    for (int v0 = 1; v0 < m; v0++) {
+// One pass of a Shell sort (D. L. Shell, 1959) over entries e[0..m): those `gap`
+// apart into order.  A step is two dependent shared-memory reads, and a thread's
+// m^2 / 4 of them on a long list were most of a dense tile's time and with it the
+// kernel's tail: passes of 13 and 4 before the last on lists over 10 (LONG: only
+// where some list is over kBucket; short lists are better off without) took the
+// splat stage at N = 64 (100k particles, 256^2 faces) from 147 to 127 us and at
+// N = 256 (1M, 1024^2) from 415 to 402.
+__device__ __forceinline__ void shell_pass(const TileSmem &S, unsigned short *e, int m, int gap) {
+    for (int v0 = gap; v0 < m; v0++) {
         const unsigned short key = e[v0];
         const unsigned long long kk = S.u.r.key[key];
-        int v = v0 - 1;
+        int v = v0 - gap;
         while (v >= 0 && S.u.r.key[e[v]] > kk) {
-            e[v + 1] = e[v];
-            v--;
+            e[v + gap] = e[v];
+            v -= gap;
         }
-        e[v + 1] = key;
+        e[v + gap] = key;
     }
+}
+
+// Sorts by key and blends the entries e[0..m) of texel q into d (upstream
+// src/render.c:135-151).
+template <bool LONG>
+__device__ __forceinline__ void blend_texel(const TileSmem &S, unsigned short *e, int m, int q, const SplatCfg &C,
+                                            const TileGeo &G, float4 &d) {
+    if (LONG && m > 10) {
+        if (m > 36) shell_pass(S, e, m, 13);
+        shell_pass(S, e, m, 4);
+    }
+    shell_pass(S, e, m, 1);
     const float invrad = C.invrad, invg = C.invg;
     const float xf = (float)(G.x0 + q % kT), yf = (float)(G.y0 + q / kT);
     for (int v = 0; v < m; v++) {
@@ -695,7 +715,7 @@ __device__ __forceinline__ void composite_window(TileSmem &S, int nw, const Spla
             if (e < kEnt) S.ent[e] = (unsigned short)s;
         });
     __syncthreads();
-    if (m) blend_texel(S, S.ent + (int)ex, m, q, C, G, d);
+    if (m) blend_texel<true>(S, S.ent + (int)ex, m, q, C, G, d);
     __syncthreads();
 }
 
@@ -814,11 +834,18 @@ __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col,
     kmin = S.u.hist[0];
     kmax = S.u.hist[1];
     __syncthreads();
+    // the records that fit a window whatever their boxes (at most 2 x 2 texels at
+    // radius 1, 3 x 3 at kWideRadius): the last window is not planned (N = 64 118 ->
+    // 113 us with buckets of a power of two of keys, found without a division)
+    const int sure = WIDE ? kRec : min(kRec, kEnt / (C.rad <= 1.0f ? 4 : 9));
+    int left = m;
     unsigned long long lo = kmin;
     while (lo <= kmax) {
-        unsigned long long top = kmax, hi;
-        for (;;) {
-            const unsigned long long span = top - lo + 1, bw = (span + kHist - 1) / kHist;
+        unsigned long long top = kmax, hi = kmax + 1;
+        while (left > sure) {
+            // a bucket is 2^sh keys
+            const int sh = max(0, 64 - __clzll(top - lo) - kHistBits);
+            const unsigned long long bw = 1ull << sh;
             for (int b = tid; b < kHist; b += kTB) S.u.hist[b] = 0;
             if (tid == 0) S.cut = kHist;
             __syncthreads();
@@ -826,7 +853,7 @@ __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col,
                 const Rec r = R[s];
                 if (r.key < lo || r.key > top) continue;
                 const int e = box_entries(rec_box(C, G, r.px, r.py));
-                if (e) atomicAdd(&S.u.hist[(r.key - lo) / bw], ((unsigned long long)(WIDE ? 0 : e) << 32) | 1ull);
+                if (e) atomicAdd(&S.u.hist[(r.key - lo) >> sh], ((unsigned long long)(WIDE ? 0 : e) << 32) | 1ull);
             }
             __syncthreads();
             // first bucket at which the running totals pass a limit
@@ -863,6 +890,7 @@ __device__ void composite_windowed(TileSmem &S, const Rec *R, const float4 *col,
             if (slot < kRec) window_put(S, slot, r, box);
         }
         __syncthreads();
+        left -= S.cut;
         const int nw = min(S.cut, kRec);
         window_colours(S, nw, col);
         __syncthreads();
@@ -963,7 +991,7 @@ __global__ void __launch_bounds__(kTB, WIDE ? 6 : 7) k_rd_tiles(SplatCfg C, cons
             __syncthreads();
             if (m <= kRec && !S.full) {
                 const int c = S.cnt[q];
-                if (c) blend_texel(S, S.bucket + q * kBucketStride, c, q, C, G, d);
+                if (c) blend_texel<false>(S, S.bucket + q * kBucketStride, c, q, C, G, d);
             } else if (m <= kRec && S.tot <= kEnt) {
                 // a texel with more than kBucket entries: pack the lists by a count scan
                 const int c = S.cnt[q];
@@ -977,7 +1005,7 @@ __global__ void __launch_bounds__(kTB, WIDE ? 6 : 7) k_rd_tiles(SplatCfg C, cons
                         if (e < kEnt) S.ent[e] = (unsigned short)s;
                     });
                 __syncthreads();
-                if (c) blend_texel(S, S.ent + st, c, q, C, G, d);
+                if (c) blend_texel<true>(S, S.ent + st, c, q, C, G, d);
             } else {
                 if (q == 0) atomicAdd(diag, 1u);
                 __syncthreads();

@@ -37,3 +37,15 @@ def test_wide_deposit_radii(gpu, orc32, R, radius):
     a = K.deposit(gpu, R, prev, pos, col, fade_steps=3, radius=radius)
     b = K.deposit(orc32, R, prev, pos, col, fade_steps=3, radius=radius)
     assert np.max(np.abs(a["faces"] - b["faces"])) <= 1e-6
+
+
+@pytest.mark.parametrize("radius", [0.75, 1.0, 1.25, 1.375])
+@pytest.mark.parametrize("n,spread", [(40, 0.01), (200, 0.02), (500, 0.02), (575, 0.05), (576, 0.05), (577, 0.05),
+                                      (900, 0.2), (1200, 0.01), (2500, 0.2)])
+def test_dense_lists(gpu, orc32, n, spread, radius):
+    """Narrower splats on a few texels: lists of 16 to several hundred entries,
+    tiles of one to several windows; bound as above."""
+    prev, pos, col = crowded(n, n + 1, spread)
+    a = K.deposit(gpu, 40, prev, pos, col, radius=radius)
+    b = K.deposit(orc32, 40, prev, pos, col, radius=radius)
+    assert np.max(np.abs(a["faces"] - b["faces"])) <= 1e-6
