@@ -724,14 +724,15 @@ __device__ __forceinline__ void composite_window(TileSmem &S, int nw, const Spla
 // leaving the records whose box meets the warp's 8 x 4 texels (wide_texel).
 // For wide splats, whose boxes hold many texels each: per (record, texel) entry
 // the lists cost a slot, an atomic and an insertion-sort step, this only the
-// blend, and a window holds any number of entries (the lists' 1728 overflow at
-// about 90 records of radius 2.5, and every window then costs two passes over the
+// blend, and a window holds any number of entries (the lists' memory is full at
+// about 150 records of radius 2.5, and every window then costs two passes over the
 // tile's records).  Bound by issue: the runs and searches take about a third, the
 // walk the rest.  200k particles on 600 x 600 faces, radius 2.5: k_rd_tiles 250 us
-// against the lists' 706; ranking by counting over all records took 330.
-// The line between lists and sorted records, whole deposits in us: 300k particles
-// on 600 x 600 faces, radius 1: 144 / 179; 1.25: 173 / 190; 1.5: 209 / 200; 20k on
-// 1000 x 1000, radius 1.5: 155 / 152; 3: 219 / 166.
+// against the lists' 706 (with windows of 1728 entries); ranking by counting over
+// all records took 330.  The line between lists and sorted records, whole deposits
+// in us: 300k particles on 600 x 600 faces, radius 1: 143 / 179; 1.25: 171 / 190;
+// 1.5: 196 / 202; 100k on 1500 x 1500, 1.5: 498 / 489; 20k on 1000 x 1000, 1.5: 148
+// / 150; 3: 198 / 166.
 constexpr float kWideRadius = 1.4f;
 __device__ __forceinline__ int wide_texel_x() { return (threadIdx.x >> 5 & 1) * 8 + (threadIdx.x & 7); }
 __device__ __forceinline__ int wide_texel_y() { return (threadIdx.x >> 6) * 4 + (threadIdx.x >> 3 & 3); }

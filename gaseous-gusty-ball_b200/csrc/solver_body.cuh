@@ -12,8 +12,8 @@
 // read between a barrier and the values that wait for it, and the window of a
 // phase holds FP32 values only.  Solve in ms, before (values, four FP64 weights
 // and three inputs of every window cell staged anew in each phase) and after:
-// N = 64 0.273, 0.242; N = 256 0.869, 0.757; N = 512 2.33, 1.92; mixed 0.852,
-// 0.775 and 2.23, 1.93.  The FP32 and FP16 roundings of every vector are unchanged.
+// N = 64 0.273, 0.230; N = 256 0.869, 0.757; N = 512 2.33, 1.92; mixed 0.852,
+// 0.757 and 2.23, 1.89.  The FP32 and FP16 roundings of every vector are unchanged.
 
 constexpr int kBlockSweepMax = 1536;  // cells of a level that one block sweeps in shared memory
 constexpr int kPBNarrow = 384;   // threads per block of the persistent kernel on small grids
@@ -27,7 +27,7 @@ constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh t
 // and 320 threads are slower from N = 128 on (0.522, 0.504).
 constexpr int kNarrowCells = 2700;
 constexpr int kWideBatchCells = 4000;  // mean cells per block of a batched launch from which its blocks are wide
-constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 256 0.756 / 0.906, 448 1.57 / 1.68, 512 1.97 / 1.92
+constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 448 1.57 / 1.68, 512 1.97 / 1.92
 constexpr int kChunk = 3072;      // cells of a stencil chunk
 constexpr double kOmegaJ = 0.8;      // upstream MG_OMEGA
 constexpr double kCorrScale = 1.0;  // upstream MG_CORR_SCALE
@@ -599,7 +599,7 @@ __device__ __forceinline__ void vcycle_block_smem(const SolveParams &P, int l0, 
 // put(row, sum_j D[row][j] b[j]) for every row of the dense map, two adjacent
 // warps per row, FP64 sums; get4(j) gives b[j..j+3] (anything past the end: the
 // map's padding columns are 0).  Bound by reading D from L2 (9.4 MB at nd =
-// 1536, 56 MB at 3750): 16-byte loads, the first kDensePre of a lane before the
+// 1536): 16-byte loads, the first kDensePre of a lane before the
 // grid barrier.  D holds FP32 values (the V-cycle it was built from works on
 // FP32 vectors), so FP32 storage loses nothing against FP64 and halves the
 // bytes.
