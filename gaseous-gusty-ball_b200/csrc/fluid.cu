@@ -667,7 +667,7 @@ GGB_EXPORT int fluid_init(Fluid *F, const CubeSphere *cs, const FluidParams *prm
         F->nlev = 0;
     }
     levels_build(solve_params(F, Pv, 0, 1), &Pv->set[0], Pv->level_mem);
-    Pv->part = (double *)dev_alloc(sizeof(double) * 4 * pcg_max_blocks());
+    Pv->part = (double *)dev_alloc(sizeof(double) * part_doubles(pcg_max_blocks()));
     Pv->bar = (GridBarrier *)dev_alloc(sizeof(GridBarrier));
     Pv->res = (SolveResult *)dev_alloc(sizeof(SolveResult));
     Pv->vmax_bits = (unsigned int *)dev_alloc(sizeof(unsigned int));

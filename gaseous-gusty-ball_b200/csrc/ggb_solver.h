@@ -1,6 +1,7 @@
 // ggb_solver.h — device descriptors of the multigrid-preconditioned CG solve.
 #pragma once
 
+#include "ggb_partials.h"
 #include "ggb_stencil.cuh"
 
 namespace ggb {
@@ -97,7 +98,7 @@ struct SolveParams {
     float *z2;           // mixed: the previous z (z / z2 ping-pong for the flexible beta)
     unsigned long long *trace;  // optional: block 0 stamps %globaltimer at phase marks
     int trace_cap;
-    double *part;        // [2][2][blocks] the blocks' sums at the last two barriers
+    double *part;        // [kPartSets][2][blocks] the blocks' sums at the last barriers
     GridBarrier *bar;
     SolveResult *res;
     // dense form of the V-cycle below the grid levels: xo_G = D b_G

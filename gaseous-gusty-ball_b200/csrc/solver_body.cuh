@@ -130,15 +130,15 @@ __device__ __noinline__ void trace_mark(int mark) {
 #define BLOCK_LOOP(c, n) for (int c = threadIdx.x; c < (n); c += blockDim.x)
 
 // Barrier of the blocks of one solve, and the sums of nv (0..2) values over all
-// their threads.  A block leaves its sums in its row of the partials (two sets
-// in turn: a set is written again only after every block has passed the barrier
-// behind its reads) and arrives at the counter; after the barrier one warp reads
-// all rows, in an order that depends on indices only, and leaves the totals in
-// s_total in every block.  With late, the totals are not read here but by the
-// next vsync called with fetch, by a second warp while the first one waits, and
-// left in s_late: a sum whose only use is the convergence test costs no round
-// trip that way.  (Arrival and sums in one message, every block polling every
-// other's slot, measured 4 us a barrier against 1.7 + 1.2.)
+// their threads.  A block leaves its sums in its row of the barrier's set of
+// partials and arrives at the counter; after the barrier one warp reads all rows,
+// in an order that depends on indices only, and leaves the totals in s_total in
+// every block.  With late, the totals are not read here but by the next vsync,
+// which must be called with fetch, by a second warp while the first one arrives
+// and waits, and left in s_late: a sum whose only use is the convergence test
+// costs no round trip that way.  What orders every read of a set before the next
+// write to it: see ggb_partials.h.  (Arrival and sums in one message, every block
+// polling every other's slot, measured 4 us a barrier against 1.7 + 1.2.)
 __device__ __forceinline__ double rows_total(const double *row, int nb, int lane) {
     double v = 0;
 #pragma unroll 5
@@ -171,7 +171,7 @@ __device__ __forceinline__ bool vsync(int nv, double v0, double v1, bool late = 
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v1 += __shfl_xor_sync(0xffffffffu, v1, o);
         }
-        double *row = sP.part + (epoch & 1) * 2 * nb;
+        double *row = sP.part + part_set(epoch) * 2 * nb;
         int ok = 1;
         if (lane == 0) {
             if (nv > 0) row[vb()] = v0;
@@ -190,7 +190,7 @@ __device__ __forceinline__ bool vsync(int nv, double v0, double v1, bool late = 
             s_epoch = epoch + 1;
         }
     } else if (warp == 1 && fetch) {
-        const double t = rows_total(sP.part + ((epoch + 1) & 1) * 2 * nb, nb, lane);
+        const double t = rows_total(sP.part + part_set(epoch - 1) * 2 * nb, nb, lane);
         if (lane == 0) s_late = t;
     }
     __syncthreads();
