@@ -1186,7 +1186,7 @@ __device__ __forceinline__ void pcg_body() {
             rz = rznew;
         }
         init = false;
-        if (it >= sP.maxit) {
+        if (!(rr > tol2) || it >= sP.maxit) {  // an rr that is NaN ends the solve, as upstream's loop condition does
             ok = true;
             break;
         }
