@@ -666,7 +666,9 @@ GGB_EXPORT int fluid_init(Fluid *F, const CubeSphere *cs, const FluidParams *prm
         Pv->nlev = 0;
         F->nlev = 0;
     }
-    levels_build(solve_params(F, Pv, 0, 1), &Pv->set[0], Pv->level_mem);
+    // A grid that is too large for the solve initialises without multigrid (only
+    // a solve of it ends with a message); it has no use for the solve's tables.
+    if (cs->N <= pcg_max_grid_n()) levels_build(solve_params(F, Pv, 0, 1), &Pv->set[0], Pv->level_mem);
     Pv->part = (double *)dev_alloc(sizeof(double) * part_doubles(pcg_max_blocks()));
     Pv->bar = (GridBarrier *)dev_alloc(sizeof(GridBarrier));
     Pv->res = (SolveResult *)dev_alloc(sizeof(SolveResult));
