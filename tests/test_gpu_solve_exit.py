@@ -1,8 +1,9 @@
 """A solve that turns NaN part way ends there, as upstream's loop does
 (src/fluid.c:290-358: it goes on while rr > tol2, which a NaN is not).
 
-psi starts as +-2e38: K psi is finite in FP64 and infinite as an FP32 residual,
-so b.b and the first r.r are finite and r.r is NaN after the first iteration.
+psi starts as +-1e38: its differences are finite in FP32, so b.b is finite and
+the first r.r is not NaN in either precision, but K psi overflows an FP32
+residual, and r.r is NaN after the first iteration.
 The iteration count has to be the restatement's."""
 import ctypes as C
 import math
@@ -20,7 +21,7 @@ SOLVE_NONFINITE, SOLVE_MAXIT = 2, 8
 
 def overflowing_state(api, g, fs):
     fs.field("omega")[:] = K.lap_exact(g.arrays()["pos"].astype(np.float64)).astype(np.float32)
-    fs.field("psi")[:] = np.where(np.arange(g.n) % 2, 2e38, -2e38).astype(np.float32)
+    fs.field("psi")[:] = np.where(np.arange(g.n) % 2, 1e38, -1e38).astype(np.float32)
 
 
 def solve(api, N, multigrid, mixed=False, maxit=60):
@@ -52,7 +53,7 @@ def test_nan_planet_does_not_hold_up_a_batch(gpu):
     fluids = [G.FluidSim(gpu, g, cg_tol=1e-6, cg_maxit=60) for _ in range(2)]
     for fs in fluids:
         fs.set_state(K.initial_velocity(gpu, g, seed=5)[0])
-    fluids[0].field("psi")[:] = np.where(np.arange(g.n) % 2, 2e38, -2e38).astype(np.float32)
+    fluids[0].field("psi")[:] = np.where(np.arange(g.n) % 2, 1e38, -1e38).astype(np.float32)
     F = (C.POINTER(gpu.T["Fluid"]) * 2)(*[C.pointer(fs.F) for fs in fluids])
     b = gpu.lib.ggb_batch_create(2, F, None, None, (C.c_double * 2)(1.0, 1.0), None)
     assert gpu.lib.ggb_batch_step(b, 1) == 0
