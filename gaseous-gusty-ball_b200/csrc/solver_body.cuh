@@ -28,6 +28,12 @@ constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh t
 constexpr int kNarrowCells = 2700;
 constexpr int kWideBatchCells = 4000;  // mean cells per block of a batched launch from which its blocks are wide
 constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 448 1.57 / 1.68, 512 1.97 / 1.92
+// Cells a thread takes at once in the vector updates of a solve without multigrid:
+// the loads of all before the stores of any, which the compiler cannot tell apart.
+// 100 iterations in us, one cell / 3: N = 64 786 / 722, 256 2031 / 1381, 512 4680 /
+// 3751.  2: 256 1414; 4: 1339, but the 512-thread kernels with multigrid spill (N =
+// 320 2 % slower).
+constexpr int kUpdate = 3;
 constexpr int kChunk = 3072;      // cells of a stencil chunk
 constexpr double kOmegaJ = 0.8;      // upstream MG_OMEGA
 constexpr double kCorrScale = 1.0;  // upstream MG_CORR_SCALE
@@ -1084,20 +1090,40 @@ __device__ __forceinline__ void pcg_body() {
             }
             if (ok) break;
         } else {
-            float *rw_ = init ? r : rn;
-            OWN_LOOP(c) {
-                double ri = ro[c];
-                if (!init) {
-                    sP.psi[c] += (float)(alpha * p[c]);
-                    ri -= alpha * Ap[c];
-                    rw_[c] = (float)ri;
+            float *rw_ = init ? r : rn, *psi = sP.psi;
+            const float *dinv = sP.L[0].dinv;
+            const int c1 = s_range[0][1], bs = blockDim.x;
+#pragma unroll 1
+            for (int c0 = s_range[0][0] + (int)threadIdx.x; c0 < c1; c0 += kUpdate * bs) {
+                float rv[kUpdate], av[kUpdate], pv[kUpdate], xv[kUpdate], dv[kUpdate];
+#pragma unroll
+                for (int u = 0; u < kUpdate; u++) {
+                    const int c = c0 + u * bs < c1 ? c0 + u * bs : c0;
+                    rv[u] = ro[c];
+                    dv[u] = __ldg(dinv + c);
+                    if (!init) {
+                        av[u] = Ap[c];
+                        pv[u] = p[c];
+                        xv[u] = psi[c];
+                    }
                 }
-                const float rc = (float)ri;
-                s += ri * ri;
-                if (!single) {
-                    const float zc = __ldg(sP.L[0].dinv + c) * rc;
-                    z[c] = zc;
-                    s2 += (double)rc * zc;
+#pragma unroll
+                for (int u = 0; u < kUpdate; u++) {
+                    const int c = c0 + u * bs;
+                    if (c >= c1) break;
+                    double ri = rv[u];
+                    if (!init) {
+                        psi[c] = xv[u] + (float)(alpha * pv[u]);
+                        ri -= alpha * av[u];
+                        rw_[c] = (float)ri;
+                    }
+                    const float rc = (float)ri;
+                    s += ri * ri;
+                    if (!single) {
+                        const float zc = dv[u] * rc;
+                        z[c] = zc;
+                        s2 += (double)rc * zc;
+                    }
                 }
             }
             if (!init) {
