@@ -628,13 +628,22 @@ __device__ __forceinline__ void vcycle_block_smem(const SolveParams &P, int l0, 
 
 // ---- the coarse end of the V-cycle ------------------------------------------
 
-// put(row, sum_j D[row][j] b[j]) for every row of the dense map, two adjacent
-// warps per row, FP64 sums; get4(j) gives b[j..j+3] (anything past the end: the
-// map's padding columns are 0).  Bound by reading D from L2 (9.4 MB at nd =
-// 1536): 16-byte loads, the first kDensePre of a lane before the
-// grid barrier.  D holds FP32 values (the V-cycle it was built from works on
-// FP32 vectors), so FP32 storage loses nothing against FP64 and halves the
-// bytes.
+// put(row, sum_j D[row][j] b[j]) for every row of the dense map, FP64 sums: each
+// half of a row over the lanes of a warp, then the two halves; get4(j) gives
+// b[j..j+3] (anything past the end: the map's padding columns are 0).  Bound by
+// reading D from L2 (9.4 MB at nd = 1536).  D holds FP32 values (the V-cycle it was
+// built from works on FP32 vectors), so FP32 storage loses nothing against FP64 and
+// halves the bytes.
+//
+// On the whole GPU a warp has one or two halves: two adjacent warps per row, 16-byte
+// loads, the first kDensePre of a lane before the grid barrier.  On a batched
+// planet's few blocks it has dozens, and each such round would be a latency, a
+// reduction and two block barriers, and convert b anew: from three rounds on
+// (BATCH) b goes to shared memory once as FP64 and every warp takes whole rows.
+// Same sums.  Batched solves in us, rounds / rows: 12 planets of N = 64 (512 threads)
+// 894 / 720; 24 of N = 64 (1024) 1292 / 1146; 60 of N = 32 2028 / 1507, 148 3924 /
+// 2819.  4 of N = 64 (384): whole rows from nine rounds on 405, from three 375.  (In
+// the kernels of single solves the rows' registers cost N = 512 1.5 %.)
 constexpr int kDensePre = 6;
 struct DenseTaps {
     float4 w[kDensePre];
@@ -648,17 +657,53 @@ __device__ __forceinline__ void dense_prefetch(DenseTaps &T) {
     for (int u = 0; u < kDensePre; u++)
         T.w[u] = j0 + lane + 32 * u < j1 ? __ldg(d + j0 + lane + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
-template <class Get4, class Put>
+template <bool BATCH, class Get4, class Put>
 __device__ __forceinline__ void dense_rows(const DenseTaps &T, Get4 get4, Put put) {
     __shared__ double s_half[32];
     const int nd = sP.nd, ld4 = sP.ld >> 2, h4 = (ld4 + 1) >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nw = (int)blockDim.x >> 5;  // even
+    const float4 *dense = reinterpret_cast<const float4 *>(sP.dense);
+    if (BATCH && nd > vnb() * nw) {
+        double2 *b0 = reinterpret_cast<double2 *>(s_win()), *b1 = b0 + ld4;
+        BLOCK_LOOP(j, ld4) {
+            const float4 b = get4(4 * j);
+            b0[j] = make_double2(b.x, b.y);
+            b1[j] = make_double2(b.z, b.w);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int row = vb() * nw + warp; row < nd; row += vnb() * nw) {
+            const float4 *d = dense + (size_t)row * ld4;
+            double v0 = 0, v1 = 0;
+            auto add = [&](double &v, float4 w, int j) {
+                const double2 p = b0[j], q = b1[j];
+                v += (double)w.x * p.x;
+                v += (double)w.y * p.y;
+                v += (double)w.z * q.x;
+                v += (double)w.w * q.y;
+            };
+#pragma unroll 3
+            for (int j = lane; j < h4; j += 32) {
+                const int k = min(j + h4, ld4 - 1);
+                const float4 w0 = __ldg(d + j), w1 = __ldg(d + k);
+                add(v0, w0, j);
+                if (j + h4 < ld4) add(v1, w1, k);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+                v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+            }
+            if (lane == 0) put(row, v0 + v1);
+        }
+        return;
+    }
     bool first = true;
 #pragma unroll 1
     for (int base = vb() * nw; base < 2 * nd; base += vnb() * nw) {
         const int part = min(base + warp, 2 * nd - 1);
         const int j1 = min(ld4, ((part & 1) + 1) * h4);
-        const float4 *d = reinterpret_cast<const float4 *>(sP.dense) + (size_t)(part >> 1) * ld4;
+        const float4 *d = dense + (size_t)(part >> 1) * ld4;
         double v = 0;
         auto add = [&](float4 w, float4 b) {
             v += (double)w.x * (double)b.x;
@@ -930,8 +975,9 @@ __device__ __forceinline__ float vscale(double rr, int n) {
 }
 
 // The whole solve of this block's planet (sP) on the block's virtual grid.
-// SWEEPS: with the sweeps of a coarsest level that has no dense map.
-template <bool MP, int TPB, bool SWEEPS>
+// SWEEPS: with the sweeps of a coarsest level that has no dense map; BATCH: the
+// virtual grid may be a few blocks.
+template <bool MP, int TPB, bool SWEEPS, bool BATCH>
 __device__ __forceinline__ void pcg_body() {
     using A = typename Prec<MP>::A;
     using V = typename Prec<MP>::V;
@@ -1176,7 +1222,7 @@ __device__ __forceinline__ void pcg_body() {
                         finish(c, as_stored<MP>(v));
                 };
                 if (sP.dense) {
-                    dense_rows(D, [&](int j) { return ldv4(cb + j); }, [&](int c, double v) { put(c, (float)v); });
+                    dense_rows<BATCH>(D, [&](int j) { return ldv4(cb + j); }, [&](int c, double v) { put(c, (float)v); });
                 } else if (!sP.coarse_on_grid) {
                     // a single small level: block 0 sweeps r in shared memory
                     if (vb() == 0) {
@@ -1288,7 +1334,7 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg(const __grid_constant__ SolvePar
         s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP, TPB, SWEEPS>();
+    pcg_body<MP, TPB, SWEEPS, false>();
 }
 
 // Many planets' solves in one cooperative launch: block b runs planet
@@ -1307,5 +1353,5 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg_batch(const SolveParams *prm, co
         s_epoch = 0;
     }
     __syncthreads();
-    pcg_body<MP, TPB, SWEEPS>();
+    pcg_body<MP, TPB, SWEEPS, true>();
 }
