@@ -326,16 +326,14 @@ GGB_EXPORT int ggb_batch_step(GGBBatch *b, int steps) {
         for (size_t g = 0; g < b->groups.size(); g++) {
             const std::vector<int> &grp = b->groups[g];
             int nb = 0;
-            long long cells = 0;
             bool sweeps = false;
             for (int i : grp) {
                 nb += b->blocks[i];
-                cells += n_cells(b, i);
                 sweeps |= b->prm_host[i].coarse_on_grid != 0;
             }
             const bool mixed = fluid_solve_mixed(b->F[grp[0]]) != 0;
-            const int alone = grp.size() == 1 && nb >= pcg_batch_capacity() ? grid_n(b, grp[0]) : 0;
-            pcg_launch_batch(b->prm_dev, b->bmap_dev + q, nb, pcg_batch_threads(cells, nb, alone), mixed, sweeps, base);
+            pcg_launch_batch(b->prm_dev, b->bmap_dev + q, nb, pcg_batch_threads(b->prm_host, grp, nb), mixed, sweeps,
+                             base);
             q += nb;
         }
         for (int i = 0; i < b->n; i++) fluid_result_queue(b->F[i]);

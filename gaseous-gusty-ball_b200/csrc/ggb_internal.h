@@ -7,6 +7,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "cubesphere.h"
 #include "fluid.h"
 #include "particles.h"
@@ -106,7 +108,7 @@ void fluid_result_velocity_queue(Fluid *F);
 int pcg_batch_capacity();
 void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, int threads, bool mixed,
                       bool sweeps, cudaStream_t s);
-int pcg_batch_threads(long long cells, int nblocks, int alone_n);
+int pcg_batch_threads(const SolveParams *prm, const std::vector<int> &planets, int nblocks);
 void render_deposit_queue(Render *r, const Particles *P);
 void render_deposit_collect(Render *r, const Particles *P);
 void particles_advect_queue(Particles *P, const CubeSphere *cs, const float *vel, const double *dt_dev);

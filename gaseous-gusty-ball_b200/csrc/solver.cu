@@ -104,10 +104,19 @@ static const void *batch_kernel(bool mixed, int threads, bool sweeps) {
     return mixed ? batch_kernel<true>(threads, sweeps) : batch_kernel<false>(threads, sweeps);
 }
 
-// Threads per block of a single solve on a grid of edge N.
-static int pcg_threads(int N) {
+// Threads per block below which a planet's solve slows down by more than its share
+// of warps: a single level that one block sweeps has a thread for every cell, with
+// its links in registers, up to 512 cells (N = 9, 486 cells: 0.18 ms, with 384
+// threads 0.74).
+static int least_threads(const SolveParams &p) {
+    return p.nlev == 1 && !p.coarse_on_grid && p.L[0].S.n > kPBNarrow ? kPB : kPBNarrow;
+}
+
+// Threads per block of a single solve.
+static int pcg_threads(const SolveParams &p) {
+    const int N = p.L[0].S.N;
     if (N >= kWideMinN) return kPBWide;
-    return 6LL * N * N <= (long long)kNarrowCells * device_sm_count() ? kPBNarrow : kPB;
+    return 6LL * N * N <= (long long)kNarrowCells * device_sm_count() ? least_threads(p) : kPB;
 }
 
 // ... of a batched launch over nblocks blocks for grids of `cells` cells in all:
@@ -116,10 +125,16 @@ static int pcg_threads(int N) {
 // edge, 8600 cells per block, mixed: 2.47 ms with 512 threads, 1.76 with 1024; 4
 // planets, 3650: 1.02 and 1.05; 2 planets, 830: 0.50 and 0.61).  alone: one planet
 // on the whole launch, with fluid_step's choice (and so its sums).
-int pcg_batch_threads(long long cells, int nblocks, int alone_n) {
-    if (alone_n > 0) return pcg_threads(alone_n);
+int pcg_batch_threads(const SolveParams *prm, const std::vector<int> &planets, int nblocks) {
+    if (planets.size() == 1 && nblocks >= pcg_batch_capacity()) return pcg_threads(prm[planets[0]]);
+    long long cells = 0;
+    int least = kPBNarrow;
+    for (int i : planets) {
+        cells += prm[i].L[0].S.n;
+        least = std::max(least, least_threads(prm[i]));
+    }
     if (cells > (long long)kWideBatchCells * nblocks) return kPBWide;
-    return cells <= (long long)kNarrowCells * nblocks ? kPBNarrow : kPB;
+    return cells <= (long long)kNarrowCells * nblocks ? least : kPB;
 }
 
 // Blocks of a launch of `kernel`.  A variant is looked at (and with lazy loading
@@ -143,7 +158,7 @@ static int blocks_resident(const void *kernel, int threads) {
 void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks) {
     SolveParams p = prm;
     void *args[] = {&p};
-    const int threads = pcg_threads(p.L[0].S.N);
+    const int threads = pcg_threads(p);
     const void *kernel = pcg_kernel(p.mixed != 0, threads, p.coarse_on_grid != 0);
     int grid = blocks_resident(kernel, threads);
     if (max_blocks > 0) grid = std::max(1, std::min(grid, max_blocks));
