@@ -119,22 +119,34 @@ static int pcg_threads(const SolveParams &p) {
     return 6LL * N * N <= (long long)kNarrowCells * device_sm_count() ? least_threads(p) : kPB;
 }
 
-// ... of a batched launch over nblocks blocks for grids of `cells` cells in all:
-// with many cells per block the chunks' loads bound a phase, not its barrier, and
-// twice the warps keep twice as many in flight (12 planets of 64 to 256 cells an
-// edge, 8600 cells per block, mixed: 2.47 ms with 512 threads, 1.76 with 1024; 4
-// planets, 3650: 1.02 and 1.05; 2 planets, 830: 0.50 and 0.61).  alone: one planet
-// on the whole launch, with fluid_step's choice (and so its sums).
+// ... of a batched launch over nblocks blocks.  With much work per block, loads and
+// arithmetic bound a phase, not its barrier, and more warps keep more in flight.
+// Work is counted in cells of the finest levels; a row of a dense map (kDenseWork
+// cells) and a cell of a swept coarsest level (kSweepWork) weigh as much as so many,
+// since few blocks have many of them: by cells alone, 45 planets of N = 32 (1870 a
+// block, 467 rows) and 6 of N = 100 (2430, no rows) would count as equals.  Batched
+// solves in us with 384 / 512 / 1024 threads, by work per block:
+//   2 planets of N = 64, 540: 323 336 453; 4 of 64, 1080: 375 383 502
+//   10 of N = 32, 1450: 403 350 489; 6 of 64, 1620: 491 437 585; 2 of 128, 1540: 517 547 673
+//   12 of 64, 3240: 843 720 755; 5 of 128, 3840: 972 880 943; 6 of 100, 5470: 2472 2372 2670
+//   2 of 256, 5520: 1187 1136 1222; 8 of 128, 6140: 1324 1187 1200; 24 of 64, 6480: 1468 1219 1146
+//   45 of 32, 6540: 1470 1210 1107; 20 of 25, 10600: 4185 4324 1815; 148 of 32, 21500: 4012 3318 2819
+// One planet on the whole launch has fluid_step's choice (and so its sums).
+constexpr int kDenseWork = 10, kSweepWork = 20;
+constexpr int kNarrowWork = 1100, kWideWork = 5800;
 int pcg_batch_threads(const SolveParams *prm, const std::vector<int> &planets, int nblocks) {
     if (planets.size() == 1 && nblocks >= pcg_batch_capacity()) return pcg_threads(prm[planets[0]]);
-    long long cells = 0;
+    long long work = 0;
     int least = kPBNarrow;
     for (int i : planets) {
-        cells += prm[i].L[0].S.n;
-        least = std::max(least, least_threads(prm[i]));
+        const SolveParams &p = prm[i];
+        work += p.L[0].S.n;
+        if (p.dense) work += (long long)kDenseWork * p.nd;
+        if (p.coarse_on_grid) work += (long long)kSweepWork * p.L[p.nlev - 1].S.n;
+        least = std::max(least, least_threads(p));
     }
-    if (cells > (long long)kWideBatchCells * nblocks) return kPBWide;
-    return cells <= (long long)kNarrowCells * nblocks ? least : kPB;
+    if (work > (long long)kWideWork * nblocks) return kPBWide;
+    return work <= (long long)kNarrowWork * nblocks ? least : kPB;
 }
 
 // Blocks of a launch of `kernel`.  A variant is looked at (and with lazy loading

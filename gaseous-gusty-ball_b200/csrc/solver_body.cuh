@@ -26,7 +26,6 @@ constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh t
 // 0.477, 192 0.626 / 0.622, 256 (2657 cells) 0.759 / 0.758, 384 1.25 / 1.34; 256
 // and 320 threads are slower from N = 128 on (0.522, 0.504).
 constexpr int kNarrowCells = 2700;
-constexpr int kWideBatchCells = 4000;  // mean cells per block of a batched launch from which its blocks are wide
 constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 448 1.57 / 1.68, 512 1.97 / 1.92
 // Cells a thread takes at once in the vector updates of a solve without multigrid:
 // the loads of all before the stores of any, which the compiler cannot tell apart.

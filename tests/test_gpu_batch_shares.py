@@ -51,8 +51,21 @@ def check(gpu, orc64, N, state):
     assert rel_l2(vel, ref["vel"]) <= 5e-5
 
 
-# with 384 threads, 40 and 127 blocks are the last that take whole rows of the 486- and 1536-row maps
+# with 512 threads (16 warps) 30 and 95 blocks are the last that take whole rows of the 486- and 1536-row maps
 @pytest.mark.parametrize("N,mixed", [(36, 0), (64, 0), (64, 1)])
-@pytest.mark.parametrize("blocks", [1, 3, 13, 40, 41, 127, 128])
+@pytest.mark.parametrize("blocks", [1, 3, 13, 30, 31, 40, 41, 95, 96, 127, 128])
 def test_dense_map_on_shares(gpu, orc64, N, mixed, blocks):
     check(gpu, orc64, N, step_batch(gpu, [N], mixed, blocks)[0])
+
+
+# launches with 384, 512 and 1024 threads a block, dense maps, swept levels and single levels side by side
+@pytest.mark.parametrize("sizes,mixed", [([64, 64], 0), ([9, 32], 0), ([17, 64, 25], 0), ([66, 32, 64, 50], 1),
+                                         ([32] * 24, 0), ([64] * 14, 1), ([25] * 12, 0)])
+def test_mixed_batches(gpu, orc64, sizes, mixed):
+    out = step_batch(gpu, sizes, mixed)
+    done = set()
+    for N, state in zip(sizes, out):
+        assert state[3] <= 1e-6
+        if N not in done:  # one planet of each size against the oracle
+            check(gpu, orc64, N, state)
+        done.add(N)
