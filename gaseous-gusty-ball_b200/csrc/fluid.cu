@@ -553,14 +553,14 @@ static void finish_levels(Fluid *F, FluidPriv *Pv) {
     }
 }
 
-void solve_trace_target(unsigned long long **buf, int *cap);
+void solve_trace_target(SolveTrace **trace, SolveTrace **stages);
 
 // Launch the solve and read back its result into F (sync).
 // Queues a solve (at most max_blocks blocks when > 0) and the copy of its
 // result; solve_collect reads the result after a synchronisation.
 static void solve_launch(Fluid *F, FluidPriv *Pv, int remove_mean, int maxit, int max_blocks) {
     SolveParams P = solve_params(F, Pv, remove_mean, maxit);
-    solve_trace_target(&P.trace, &P.trace_cap);
+    solve_trace_target(&P.trace, &P.stages);
     cudaStream_t s = stream();
     stage_begin(ST_SOLVE);
     pcg_launch(P, s, max_blocks);

@@ -80,6 +80,14 @@ struct SolveResult {
     unsigned long long ns;  // device time of the solve (%globaltimer, block 0 of the solve)
 };
 
+// Diagnostic records of a solve (device memory): up to cap (mark, ns) pairs.
+struct SolveTrace {
+    int n, cap;
+    int all;  // stage marks: 1 from every block, 0 from the launch's block 0
+    int pad;
+    unsigned long long rec[1][2];  // [cap]
+};
+
 struct SolveParams {
     int mixed;           // 1: V-cycle vectors in FP16 with FP32 accumulation, flexible (Polak-Ribiere) CG;
                          //    0: FP32 vectors, FP64 accumulation
@@ -96,8 +104,8 @@ struct SolveParams {
     float *omega, *psi;
     float *r, *r2, *p, *p2, *Ap, *z;  // level-0 CG vectors (r / p ping-pong)
     float *z2;           // mixed: the previous z (z / z2 ping-pong for the flexible beta)
-    unsigned long long *trace;  // optional: block 0 stamps %globaltimer at phase marks
-    int trace_cap;
+    SolveTrace *trace;   // optional: block 0 of the solve stamps %globaltimer at phase marks
+    SolveTrace *stages;  // optional: ... at the start and end of every stencil phase
     double *part;        // [kPartSets][2][blocks] the blocks' sums at the last barriers
     GridBarrier *bar;
     SolveResult *res;

@@ -34,9 +34,9 @@
 //     fixed linear map, precomputed once as a dense matrix and applied by all
 //     blocks from L2.
 #include <algorithm>
+#include <cstddef>
 #include <cstdio>
 #include <mutex>
-#include <type_traits>
 #include <vector>
 
 #include "ggb_internal.h"
@@ -67,11 +67,12 @@ __global__ void __launch_bounds__(kPB, 1) k_dense_columns(SolveParams P, int l0,
 
 // ---------------------------------------------------------------- host
 
-static unsigned long long *g_trace_dev = nullptr;
+static SolveTrace *g_trace = nullptr, *g_stages = nullptr;
 static int g_trace_cap = 0;
-void solve_trace_target(unsigned long long **buf, int *cap) {
-    *buf = g_trace_dev;
-    *cap = g_trace_cap;
+static bool g_stages_on = false;
+void solve_trace_target(SolveTrace **trace, SolveTrace **stages) {
+    *trace = g_trace;
+    *stages = g_stages_on ? g_stages : nullptr;
 }
 
 int pcg_max_blocks() { return device_sm_count(); }
@@ -81,27 +82,9 @@ int pcg_max_blocks() { return device_sm_count(); }
 // bound is the one fluid_init's callers have always had).
 int pcg_max_grid_n() { return 1535; }
 
-template <bool MP>
-static const void *pcg_kernel(int threads, bool sweeps) {
-    if (threads == kPBWide)
-        return sweeps ? (const void *)k_pcg<MP, kPBWide, true> : (const void *)k_pcg<MP, kPBWide, false>;
-    if (threads == kPBNarrow)
-        return sweeps ? (const void *)k_pcg<MP, kPBNarrow, true> : (const void *)k_pcg<MP, kPBNarrow, false>;
-    return sweeps ? (const void *)k_pcg<MP, kPB, true> : (const void *)k_pcg<MP, kPB, false>;
-}
-static const void *pcg_kernel(bool mixed, int threads, bool sweeps) {
-    return mixed ? pcg_kernel<true>(threads, sweeps) : pcg_kernel<false>(threads, sweeps);
-}
-template <bool MP>
-static const void *batch_kernel(int threads, bool sweeps) {
-    if (threads == kPBWide)
-        return sweeps ? (const void *)k_pcg_batch<MP, kPBWide, true> : (const void *)k_pcg_batch<MP, kPBWide, false>;
-    if (threads == kPBNarrow)
-        return sweeps ? (const void *)k_pcg_batch<MP, kPBNarrow, true> : (const void *)k_pcg_batch<MP, kPBNarrow, false>;
-    return sweeps ? (const void *)k_pcg_batch<MP, kPB, true> : (const void *)k_pcg_batch<MP, kPB, false>;
-}
-static const void *batch_kernel(bool mixed, int threads, bool sweeps) {
-    return mixed ? batch_kernel<true>(threads, sweeps) : batch_kernel<false>(threads, sweeps);
+static const void *pcg_kernel(bool mixed, int threads, bool sweeps, bool batch) {
+    if (mixed) return sweeps ? kernel_of<true, true>(threads, batch) : kernel_of<true, false>(threads, batch);
+    return sweeps ? kernel_of<false, true>(threads, batch) : kernel_of<false, false>(threads, batch);
 }
 
 // Threads per block below which a planet's solve slows down by more than its share
@@ -171,7 +154,7 @@ void pcg_launch(const SolveParams &prm, cudaStream_t s, int max_blocks) {
     SolveParams p = prm;
     void *args[] = {&p};
     const int threads = pcg_threads(p);
-    const void *kernel = pcg_kernel(p.mixed != 0, threads, p.coarse_on_grid != 0);
+    const void *kernel = pcg_kernel(p.mixed != 0, threads, p.coarse_on_grid != 0, false);
     int grid = blocks_resident(kernel, threads);
     if (max_blocks > 0) grid = std::max(1, std::min(grid, max_blocks));
     GGB_CHECK(cudaMemsetAsync(&p.bar->count, 0, sizeof(unsigned int), s));
@@ -189,7 +172,7 @@ int pcg_batch_capacity() { return device_sm_count(); }
 // planets' barrier counters must be zero.
 void pcg_launch_batch(const SolveParams *dev_prm, const int4 *dev_bmap, int nblocks, int threads, bool mixed,
                       bool sweeps, cudaStream_t s) {
-    const void *k = batch_kernel(mixed, threads, sweeps);
+    const void *k = pcg_kernel(mixed, threads, sweeps, true);
     blocks_resident(k, threads);
     void *args[] = {(void *)&dev_prm, (void *)&dev_bmap};
     GGB_CHECK(cudaLaunchCooperativeKernel(k, dim3(nblocks), dim3(threads), args, kStageBytes, s));
@@ -282,27 +265,42 @@ GGB_EXPORT int ggb_barrier_timeout_probe(double limit_ms, double *elapsed_ms) {
     return ok ? 0 : 1;
 }
 
+static size_t trace_bytes(int cap) { return sizeof(ggb::SolveTrace) + 2 * sizeof(unsigned long long) * (size_t)cap; }
+
+// Empties a trace buffer and sets its size and mode.
+static void trace_reset(ggb::SolveTrace *t, int cap, int all) {
+    ggb::SolveTrace head{};
+    head.cap = cap;
+    head.all = all;
+    GGB_CHECK(cudaMemcpy(t, &head, offsetof(ggb::SolveTrace, rec), cudaMemcpyHostToDevice));
+}
+
+// Copies out up to cap records; their number.
+static int trace_read(const ggb::SolveTrace *t, unsigned long long *out, int cap) {
+    ggb::SolveTrace head{};
+    GGB_CHECK(cudaMemcpy(&head, t, offsetof(ggb::SolveTrace, rec), cudaMemcpyDeviceToHost));
+    const int n = std::min(std::min(head.n, head.cap), cap);
+    if (n > 0) GGB_CHECK(cudaMemcpy(out, t->rec, 2 * sizeof(unsigned long long) * (size_t)n, cudaMemcpyDeviceToHost));
+    return n;
+}
+
 // Diagnostics: the next solves record up to `cap` (mark, time in ns) pairs from
 // block 0 (cap = 0 turns it off); ggb_solve_trace copies them out and returns
 // how many were recorded.
 GGB_EXPORT void ggb_solve_trace_enable(int cap) {
     using namespace ggb;
     sync();
-    dev_free(g_trace_dev);
-    g_trace_dev = cap > 0 ? (unsigned long long *)dev_alloc(sizeof(unsigned long long) * 2 * cap) : nullptr;
+    dev_free(g_trace);
+    g_trace = cap > 0 ? (SolveTrace *)dev_alloc(trace_bytes(cap)) : nullptr;
     g_trace_cap = cap > 0 ? cap : 0;
-    int zero = 0;
-    GGB_CHECK(cudaMemcpyToSymbol(g_trace_n, &zero, sizeof(int)));
+    sync();
+    if (g_trace) trace_reset(g_trace, g_trace_cap, 0);
 }
 
 GGB_EXPORT int ggb_solve_trace(unsigned long long *out, int cap) {
     using namespace ggb;
     sync();
-    int n = 0;
-    GGB_CHECK(cudaMemcpyFromSymbol(&n, g_trace_n, sizeof(int)));
-    n = n < cap ? n : cap;
-    if (n > 0) GGB_CHECK(cudaMemcpy(out, g_trace_dev, sizeof(unsigned long long) * 2 * n, cudaMemcpyDeviceToHost));
-    return n;
+    return g_trace ? trace_read(g_trace, out, cap) : 0;
 }
 
 // Diagnostics: enable = 1 makes block 0 of the next solves stamp the start
@@ -311,22 +309,14 @@ GGB_EXPORT int ggb_solve_trace(unsigned long long *out, int cap) {
 // out up to cap records, returning their number.
 GGB_EXPORT int ggb_stage_trace(int enable, unsigned long long *out, int cap) {
     using namespace ggb;
+    constexpr int kRecords = 4096;
     sync();
-    static unsigned long long *buf = nullptr;
-    int n = 0;
-    if (!enable) {
-        unsigned long long *null = nullptr;
-        GGB_CHECK(cudaMemcpyFromSymbol(&n, g_stage_trace_n, sizeof(int)));
-        GGB_CHECK(cudaMemcpyToSymbol(g_stage_trace, &null, sizeof(null)));
-        n = n < cap ? n : cap;
-        n = n < 4096 ? n : 4096;
-        if (n > 0 && buf) GGB_CHECK(cudaMemcpy(out, buf, sizeof(unsigned long long) * 2 * n, cudaMemcpyDeviceToHost));
-        return n;
+    g_stages_on = enable != 0;
+    if (!enable) return g_stages ? trace_read(g_stages, out, cap) : 0;
+    if (!g_stages) {
+        g_stages = (SolveTrace *)dev_alloc(trace_bytes(kRecords));
+        sync();
     }
-    if (!buf) buf = (unsigned long long *)dev_alloc(sizeof(unsigned long long) * 2 * 4096);
-    const int all = enable == 2;
-    GGB_CHECK(cudaMemcpyToSymbol(g_stage_trace, &buf, sizeof(buf)));
-    GGB_CHECK(cudaMemcpyToSymbol(g_stage_trace_n, &n, sizeof(int)));
-    GGB_CHECK(cudaMemcpyToSymbol(g_stage_trace_all, &all, sizeof(int)));
+    trace_reset(g_stages, kRecords, enable == 2);
     return 0;
 }

@@ -109,21 +109,26 @@ __device__ __forceinline__ float *s_win() { return reinterpret_cast<float *>(s_d
 
 __device__ __forceinline__ float *s_pool() { return s_win() + kWinCap; }
 
-// Phase trace (diagnostics): block 0, thread 0 records (mark, %globaltimer).
-__device__ int g_trace_n;
-__device__ __noinline__ void trace_mark(int mark) {
-    if (vb() == 0 && threadIdx.x == 0) {
-        const int k = g_trace_n;
-        if (k < sP.trace_cap) {
-            sP.trace[2 * k] = (unsigned long long)mark;
-            sP.trace[2 * k + 1] = globaltimer_ns();
-            g_trace_n = k + 1;
-        }
+// Traces (diagnostics): (mark, %globaltimer) pairs into a SolveTrace, whose pointer
+// is among the parameters, so that an untraced solve only tests it in shared memory.
+__device__ __noinline__ void trace_mark(SolveTrace *t, unsigned long long mark) {
+    if (threadIdx.x != 0) return;
+    const int k = atomicAdd(&t->n, 1);
+    if (k < t->cap) {
+        t->rec[k][0] = mark;
+        t->rec[k][1] = globaltimer_ns();
     }
 }
-#define TRACE(mark)                    \
-    do {                               \
-        if (sP.trace) trace_mark(mark); \
+// the schedule's phases, from block 0
+#define TRACE(mark)                                                    \
+    do {                                                               \
+        if (sP.trace && vb() == 0) trace_mark(sP.trace, (mark));       \
+    } while (0)
+// the stencil phases' start (1) and end (2), from block 0 of the launch or all blocks
+#define STAGE_MARK(mark)                                                                              \
+    do {                                                                                              \
+        if (sP.stages && (sP.stages->all || blockIdx.x == 0))                                         \
+            trace_mark(sP.stages, (mark) | (sP.stages->all ? (unsigned long long)blockIdx.x << 16 : 0)); \
     } while (0)
 
 // GRID_LOOP: over the block's virtual grid (only inside k_pcg / k_pcg_batch,
@@ -238,28 +243,6 @@ __device__ __forceinline__ void block_range(int n, int &c0, int &c1) {
     c1 = (int)(((long long)n * (vb() + 1)) / vnb());
 }
 
-__device__ unsigned long long *g_stage_trace;  // diagnostics: block 0 stamps the stencil phases
-__device__ int g_stage_trace_n;
-__device__ int g_stage_trace_all;  // 1: every block records, mark | block << 16
-__device__ __noinline__ void stage_mark(int mark) {
-    unsigned long long *t = g_stage_trace;
-    if (!t || threadIdx.x != 0) return;
-    if (g_stage_trace_all) {
-        const int k = atomicAdd(&g_stage_trace_n, 1);
-        if (k < 4096) {
-            t[2 * k] = (unsigned long long)(mark | (blockIdx.x << 16));
-            t[2 * k + 1] = globaltimer_ns();
-        }
-    } else if (blockIdx.x == 0) {
-        int k = g_stage_trace_n;
-        if (k < 4096) {
-            t[2 * k] = (unsigned long long)mark;
-            t[2 * k + 1] = globaltimer_ns();
-            g_stage_trace_n = k + 1;
-        }
-    }
-}
-
 __device__ __forceinline__ void cp_async16(float *dst, const float *src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
@@ -372,7 +355,7 @@ __device__ __forceinline__ void stencil_phase(int l, RingPre &R, Load load, Cell
     const StencilDev &S = L.S;
     const int N = S.N, n = S.n, bs = blockDim.x, tid = threadIdx.x, lane = tid & 31;
     const int c0 = s_range[l][0], c1 = s_range[l][1];
-    stage_mark(1);
+    STAGE_MARK(1);
     const int total = 48 * S.nring, stride = 32 * vwarps();
 #pragma unroll 1
     for (int e0 = 32 * vwarp(); e0 < total; e0 += stride) {
@@ -426,7 +409,7 @@ __device__ __forceinline__ void stencil_phase(int l, RingPre &R, Load load, Cell
                 cell(c, x[c], apply_window<A>(c, N, x, wE, wE + cap, wE + 2 * cap, wE + 3 * cap));
         __syncthreads();
     }
-    stage_mark(2);
+    STAGE_MARK(2);
 }
 
 // ---- sparse rows ------------------------------------------------------------
@@ -1353,4 +1336,14 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg_batch(const SolveParams *prm, co
     }
     __syncthreads();
     pcg_body<MP, TPB, SWEEPS, true>();
+}
+
+// The kernel of a precision and coarse end at one of the block sizes.
+template <bool MP, bool SWEEPS>
+const void *kernel_of(int threads, bool batch) {
+    if (threads == kPBWide)
+        return batch ? (const void *)k_pcg_batch<MP, kPBWide, SWEEPS> : (const void *)k_pcg<MP, kPBWide, SWEEPS>;
+    if (threads == kPBNarrow)
+        return batch ? (const void *)k_pcg_batch<MP, kPBNarrow, SWEEPS> : (const void *)k_pcg<MP, kPBNarrow, SWEEPS>;
+    return batch ? (const void *)k_pcg_batch<MP, kPB, SWEEPS> : (const void *)k_pcg<MP, kPB, SWEEPS>;
 }
