@@ -44,7 +44,15 @@
 
 namespace ggb {
 
+namespace {
 #include "solver_body.cuh"
+}
+
+// solver_plain.cu, solver_plain_sweeps.cu, solver_mixed.cu, solver_mixed_sweeps.cu
+const void *pcg_kernel_plain(int threads, bool batch);
+const void *pcg_kernel_plain_sweeps(int threads, bool batch);
+const void *pcg_kernel_mixed(int threads, bool batch);
+const void *pcg_kernel_mixed_sweeps(int threads, bool batch);
 
 // ---- setup kernels -------------------------------------------------------
 
@@ -83,8 +91,8 @@ int pcg_max_blocks() { return device_sm_count(); }
 int pcg_max_grid_n() { return 1535; }
 
 static const void *pcg_kernel(bool mixed, int threads, bool sweeps, bool batch) {
-    if (mixed) return sweeps ? kernel_of<true, true>(threads, batch) : kernel_of<true, false>(threads, batch);
-    return sweeps ? kernel_of<false, true>(threads, batch) : kernel_of<false, false>(threads, batch);
+    if (mixed) return sweeps ? pcg_kernel_mixed_sweeps(threads, batch) : pcg_kernel_mixed(threads, batch);
+    return sweeps ? pcg_kernel_plain_sweeps(threads, batch) : pcg_kernel_plain(threads, batch);
 }
 
 // Threads per block below which a planet's solve slows down by more than its share

@@ -1,6 +1,9 @@
 // solver_body.cuh — the device code of the persistent solve kernels k_pcg /
-// k_pcg_batch (constants, stencil phases, V-cycle, PCG body), included by
-// solver.cu inside its namespace.
+// k_pcg_batch (constants, stencil phases, V-cycle, PCG body), included inside an
+// unnamed namespace by solver.cu (set-up kernels and the host side) and by
+// solver_{plain,mixed}{,_sweeps}.cu, which compile the solve kernels of one
+// precision and coarse end each: a module is brought to the device as a whole, and
+// all 24 kernels in one cost a program's first call 18 ms.
 //
 // Upstream: src/fluid.c:41-160 (multigrid), :264-275 (mean), :290-358 (PCG).
 //
