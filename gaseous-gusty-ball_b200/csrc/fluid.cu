@@ -465,7 +465,6 @@ static void build_levels(Fluid *F, FluidPriv *Pv) {
     }
 }
 
-constexpr int kBlockLevelMax = 1536;  // levels up to N=16 form the dense coarse map (a single level: one block sweeps it)
 static SolveParams solve_params(Fluid *F, FluidPriv *Pv, int remove_mean, int maxit) {
     if (F->cs->N > pcg_max_grid_n())
         fail_msg("grids with N > %d exceed the solve kernel's staged window (N = %d)", pcg_max_grid_n(), F->cs->N);

@@ -8,6 +8,10 @@ namespace ggb {
 
 constexpr int kMaxLev = 12;
 
+// Cells of a level up to which the levels from it down form the dense coarse map,
+// and a single level is swept by one block in shared memory (N <= 16).
+constexpr int kBlockLevelMax = 1536;
+
 // Sparse rows of (index, weight bits) taps: step s of row r is tap[s * rows + r].
 // glen: the steps that each 32 rows need (stored steps past a row's own taps
 // have weight 0).

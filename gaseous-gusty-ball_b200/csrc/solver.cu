@@ -85,10 +85,8 @@ void solve_trace_target(SolveTrace **trace, SolveTrace **stages) {
 
 int pcg_max_blocks() { return device_sm_count(); }
 
-// Largest grid edge a solve accepts (the stencil window, kWinCap cells, must
-// hold a block of threads' worth of cells between its two halos of N + 1; the
-// bound is the one fluid_init's callers have always had).
-int pcg_max_grid_n() { return 1535; }
+// Largest grid edge a solve accepts: a window holds a chunk and two halos of N + 1.
+int pcg_max_grid_n() { return kMaxN; }
 
 static const void *pcg_kernel(bool mixed, int threads, bool sweeps, bool batch) {
     if (mixed) return sweeps ? pcg_kernel_mixed_sweeps(threads, batch) : pcg_kernel_mixed(threads, batch);

@@ -18,7 +18,6 @@
 // N = 64 0.273, 0.230; N = 256 0.869, 0.757; N = 512 2.33, 1.92; mixed 0.852,
 // 0.757 and 2.23, 1.89.  The FP32 and FP16 roundings of every vector are unchanged.
 
-constexpr int kBlockSweepMax = 1536;  // cells of a level that one block sweeps in shared memory
 constexpr int kPBNarrow = 384;   // threads per block of the persistent kernel on small grids
 constexpr int kPB = 512;         // ... on ordinary ones
 constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh the phases' latency
@@ -45,7 +44,8 @@ constexpr double kCorrScale = 1.0;  // upstream MG_CORR_SCALE
 constexpr int kMaxN = 1535;
 constexpr int kWinCap = (kChunk + 2 * kMaxN + 2 + 3) & ~3;  // whole 16-byte groups: the pool follows
 static_assert(kWinCap >= 2 * kSweepSlots, "two buffers of a part's values");
-static_assert(kWinCap >= 3 * kBlockSweepMax, "x, xo and b of a level that one block sweeps");
+static_assert(kWinCap >= 3 * kBlockLevelMax, "x, xo and b of a level that one block sweeps");
+static_assert(kWinCap >= 2 * ((kBlockLevelMax + 3) & ~3), "b of the dense map in FP64");
 constexpr int kSlotPool = 34816;
 static_assert(kSlotPool >= 4 * (kChunk + 2 * kMaxN + 2 + 8), "a chunk's slot weights fit");
 constexpr size_t kStageBytes = (kWinCap + (size_t)kSlotPool) * sizeof(float);
