@@ -109,13 +109,7 @@ __device__ __forceinline__ double apply_k(const StencilDev &S, int c, double xc,
     return s + ring_extras(S, f, i, j, xc, X_);
 }
 
-// Boundary-ring cells in cell order: the number of ring cells with index
-// below c (c in [0, n]), and the cell of ring rank R.
-__device__ __forceinline__ int ring_rank_below(int c, int N, int nring) {
-    int f, i, j;
-    cell_fij(c, N, f, i, j);
-    return f * nring + ring_rank_in_face(i, j, N);
-}
+// The boundary-ring cell of ring rank R (the rank is in cell order).
 __device__ __forceinline__ void ring_cell_of_rank(int R, int N, int nring, int &f, int &i, int &j) {
     f = R / nring;
     const int q = R - f * nring;

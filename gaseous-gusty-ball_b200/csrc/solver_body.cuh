@@ -135,9 +135,8 @@ __device__ __noinline__ void trace_mark(SolveTrace *t, unsigned long long mark) 
     } while (0)
 
 // GRID_LOOP: over the block's virtual grid (only inside k_pcg / k_pcg_batch,
-// which set it); KERNEL_LOOP: over the launch's real grid (set-up kernels).
+// which set it).
 #define GRID_LOOP(c, n) for (int c = vb() * blockDim.x + threadIdx.x; c < (n); c += vnb() * blockDim.x)
-#define KERNEL_LOOP(c, n) for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < (n); c += gridDim.x * blockDim.x)
 // OWN_LOOP: the cells of this block's level-0 range
 #define OWN_LOOP(c) for (int c = s_range[0][0] + (int)threadIdx.x; c < s_range[0][1]; c += blockDim.x)
 #define BLOCK_LOOP(c, n) for (int c = threadIdx.x; c < (n); c += blockDim.x)
