@@ -410,7 +410,7 @@ static StencilDev stencil_of(const GridTables *t) {
     s.N = t->N;
     s.n = t->n;
     s.nring = t->nring;
-    s.rN = ((1ull << 40) + t->N - 1) / t->N;
+    s.rN = div_factor(t->N);
     s.wslot = t->wslot;
     s.wpad = t->wpad;
     s.pad = t->N + 1;

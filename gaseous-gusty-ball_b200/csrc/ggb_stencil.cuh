@@ -7,12 +7,13 @@
 #include <cuda_fp16.h>
 
 #include "ggb_device.cuh"
+#include "ggb_divide.h"
 
 namespace ggb {
 
 struct StencilDev {
     int N, n, nring;
-    unsigned long long rN;  // ceil(2^40 / N)
+    unsigned long long rN;  // div_factor(N)
     const float *wslot;   // [4][n]: E, N, NE, NW weights (0 = no link)
     const float *wpad;    // the four planes with at least pad zeros before and after each, plane stride wplane (x 4)
     int pad, wplane;
@@ -35,12 +36,11 @@ __device__ __forceinline__ void cell_fij(int c, int N, int &f, int &i, int &j) {
     i = rem - j * N;
 }
 
-// cell_fij for a level's stencil: the divisions as multiplications by rN =
-// ceil(2^40 / N) (exact: c < 6 N^2 <= 2^24 and N <= 1535, so c N < 2^40), which take a
+// cell_fij for a level's stencil: the divisions as multiplications, which take a
 // fraction of an integer division's instructions.
 __device__ __forceinline__ void cell_fij(const StencilDev &S, int c, int &f, int &i, int &j) {
-    const int row = (int)(((unsigned long long)(unsigned)c * S.rN) >> 40);  // c / N
-    f = (int)(((unsigned long long)(unsigned)row * S.rN) >> 40);
+    const int row = div_by((unsigned)c, S.rN);
+    f = div_by((unsigned)row, S.rN);
     i = c - row * S.N;
     j = row - f * S.N;
 }
