@@ -331,11 +331,7 @@ void sweep_parts_build(const StencilDev &S, int blocks, SweepParts *out, std::ve
     unsigned short *nb = (unsigned short *)dev_alloc(sizeof(unsigned short) * parts * kMaxNb * kSweepSlots);
     float *w = (float *)dev_alloc(sizeof(float) * parts * kMaxNb * kSweepSlots);
     for (void *p : {(void *)count, (void *)cell, (void *)nb, (void *)w}) mem.push_back(p);
-    static bool attr = false;
-    if (!attr) {
-        GGB_CHECK(cudaFuncSetAttribute(k_sweep_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr = true;
-    }
+    GGB_CHECK(cudaFuncSetAttribute(k_sweep_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     k_sweep_parts<<<parts, kPartThreads, smem, s>>>(S, tx, ty, count, cell, nb, w);
     GGB_LAUNCHED();
     std::vector<int> host((size_t)parts * (kSweepDepth + 1));
