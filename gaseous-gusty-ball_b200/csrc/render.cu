@@ -729,10 +729,17 @@ __device__ __forceinline__ void composite_window(TileSmem &S, int nw, const Spla
 // tile's records).  Bound by issue: the runs and searches take about a third, the
 // walk the rest.  200k particles on 600 x 600 faces, radius 2.5: k_rd_tiles 250 us
 // against the lists' 706 (with windows of 1728 entries); ranking by counting over
-// all records took 330.  The line between lists and sorted records, whole deposits
-// in us: 300k particles on 600 x 600 faces, radius 1: 143 / 179; 1.25: 171 / 190;
-// 1.5: 196 / 202; 100k on 1500 x 1500, 1.5: 498 / 489; 20k on 1000 x 1000, 1.5: 148
-// / 150; 3: 198 / 166.
+// all records took 330.
+//
+// The line between lists and sorted records, whole deposits in us (lists / sorted):
+// 200k particles on 256 x 256 faces: radius 1.42 211 / 237, 1.5 233 / 246, 1.6 262 /
+// 257, 1.75 323 / 262; 200k on 1024 x 1024: 448 / 466, 473 / 477, 541 / 486, 610 /
+// 504; 20k on 600 x 600: 122 / 122, 125 / 121, 136 / 122, 139 / 122.  Where tiles are
+// crowded the lists lose far sooner: 1M on 256 x 256: 1944 / 1487, 2079 / 1514; 200k
+// on 64 x 64: 1275 / 758, 1361 / 771; there radius 1 is the lists' (1M on 256 x 256
+// 1.1 ms, N = 256 stage 416 / 610).  1.4 gives up to 12 % on the first kind below 1.6
+// for 25 to 45 % on the second; and up to it a box has at most 3 x 3 texels, which
+// composite_windowed counts on for lists.
 constexpr float kWideRadius = 1.4f;
 __device__ __forceinline__ int wide_texel_x() { return (threadIdx.x >> 5 & 1) * 8 + (threadIdx.x & 7); }
 __device__ __forceinline__ int wide_texel_y() { return (threadIdx.x >> 6) * 4 + (threadIdx.x >> 3 & 3); }
