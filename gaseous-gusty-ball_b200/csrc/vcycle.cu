@@ -150,69 +150,102 @@ __global__ void k_round_half(size_t n, const float *src, float *dst) {
         dst[i] = __half2float(__float2half_rn(src[i]));
 }
 
-static void ring_links(const StencilDev &S, int half, LevelSet *out, int l, std::vector<void *> &mem, int *bad) {
-    int2 *link = (int2 *)dev_alloc(sizeof(int2) * kMaxNb * 6 * (size_t)S.nring);
-    int *cell = (int *)dev_alloc(sizeof(int) * 6 * (size_t)S.nring);
-    mem.push_back(link);
-    mem.push_back(cell);
+static void ring_links(const StencilDev &S, int half, int2 *link, int *cell, LevelSet *out, int l, int *bad) {
     k_ring_links<<<setup_blocks(6 * S.nring), kSB, 0, stream()>>>(S, half, link, cell, bad);
     GGB_LAUNCHED();
     out->ring_link[l] = link;
     out->ring_cell[l] = cell;
 }
+static size_t ring_link_bytes(const StencilDev &S) { return sizeof(int2) * kMaxNb * 6 * (size_t)S.nring; }
+static size_t ring_cell_bytes(const StencilDev &S) { return sizeof(int) * 6 * (size_t)S.nring; }
+
+// The places of several arrays in one allocation: at least one call of the
+// allocator a level was most of this set-up's time.
+struct Layout {
+    size_t bytes = 0;
+    size_t take(size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) & ~(size_t)255;
+        return at;
+    }
+};
 
 // The plain solve's level data (levels 0..nlev_grid of P; level 0's ring links
 // for every fluid).  The device arrays go to mem.
 void levels_build(const SolveParams &P, LevelSet *out, std::vector<void *> &mem) {
     cudaStream_t s = stream();
     const int G = P.nlev_grid;
-    int *scratch = (int *)dev_alloc(sizeof(int) * (2 * kMaxLev + 1));
-    for (int l = 0; l < std::max(G, 1); l++) ring_links(P.L[l].S, 0, out, l, mem, scratch + 2 * kMaxLev);
-    for (int l = 0; l < G; l++) {
-        k_check_structured<<<setup_blocks(P.L[l].S.n), kSB, 0, s>>>(P.L[l], P.L[l + 1].S, scratch + 2 * l);
-        GGB_LAUNCHED();
+    struct Host {
+        int irregular[kMaxLev];                     // rows and taps off the index pattern
+        int most[kMaxLev], most_ring[kMaxLev];      // longest row of R: of all, of the coarse ring's
+        int bad;                                    // ring cells of too many links
+    } host = {};
+    struct At {
+        size_t link, cell, rw16, r, b, xo, tap, glen;
+    } at[kMaxLev] = {};
+    Layout first;
+    const size_t scratch_at = first.take(sizeof(Host));
+    for (int l = 0; l < std::max(G, 1); l++) {
+        at[l].link = first.take(ring_link_bytes(P.L[l].S));
+        at[l].cell = first.take(ring_cell_bytes(P.L[l].S));
     }
-    int host[2 * kMaxLev + 1] = {};
-    GGB_CHECK(cudaMemcpyAsync(host, scratch, sizeof(host), cudaMemcpyDeviceToHost, s));
-    GGB_CHECK(cudaStreamSynchronize(s));
-    if (host[2 * kMaxLev]) fail_msg("multigrid set-up: a ring cell of more than %d links", kMaxNb);
+    for (int l = 0; l < G; l++) {
+        const size_t nc = P.L[l + 1].S.n;
+        at[l].rw16 = first.take(sizeof(float) * 16 * nc);
+        at[l].r = first.take(sizeof(float) * (size_t)P.L[l].S.n);
+        at[l].b = first.take(sizeof(float) * (nc + 8));
+        at[l].xo = first.take(sizeof(float) * (nc + 8));
+    }
+    unsigned char *const vectors = (unsigned char *)dev_alloc(first.bytes);
+    mem.push_back(vectors);
+    Host *scratch = (Host *)(vectors + scratch_at);
+    for (int l = 0; l < std::max(G, 1); l++)
+        ring_links(P.L[l].S, 0, (int2 *)(vectors + at[l].link), (int *)(vectors + at[l].cell), out, l, &scratch->bad);
     for (int l = 0; l < G; l++) {
         const StencilDev &C = P.L[l + 1].S;
-        out->rst[l].rows = host[2 * l] == 0 ? 6 * C.nring : C.n;
-        k_row_len<<<setup_blocks(out->rst[l].rows), kSB, 0, s>>>(P.L[l], C, host[2 * l] == 0, out->rst[l].rows,
-                                                               scratch + 2 * l + 1);
+        k_check_structured<<<setup_blocks(P.L[l].S.n), kSB, 0, s>>>(P.L[l], C, &scratch->irregular[l]);
         GGB_LAUNCHED();
+        k_row_len<<<setup_blocks(C.n), kSB, 0, s>>>(P.L[l], C, 0, C.n, &scratch->most[l]);
+        GGB_LAUNCHED();
+        k_row_len<<<setup_blocks(6 * C.nring), kSB, 0, s>>>(P.L[l], C, 1, 6 * C.nring, &scratch->most_ring[l]);
+        GGB_LAUNCHED();
+        out->r[l] = vectors + at[l].r;
+        out->b[l + 1] = vectors + at[l].b;
+        out->xo[l + 1] = vectors + at[l].xo;
     }
-    GGB_CHECK(cudaMemcpyAsync(host, scratch, sizeof(host), cudaMemcpyDeviceToHost, s));
+    GGB_CHECK(cudaMemcpyAsync(&host, scratch, sizeof(host), cudaMemcpyDeviceToHost, s));
     GGB_CHECK(cudaStreamSynchronize(s));
+    if (host.bad) fail_msg("multigrid set-up: a ring cell of more than %d links", kMaxNb);
+    Layout second;
     for (int l = 0; l < G; l++) {
         const StencilDev &C = P.L[l + 1].S;
-        const int ring = host[2 * l] == 0;
+        const bool ring = host.irregular[l] == 0;
         SparseOp &op = out->rst[l];
-        op.steps = std::max(1, host[2 * l + 1]);
+        op.rows = ring ? 6 * C.nring : C.n;
+        op.steps = std::max(1, ring ? host.most_ring[l] : host.most[l]);
         if (op.steps > 255) fail_msg("multigrid set-up: a row of %d taps", op.steps);
-        int2 *tap = (int2 *)dev_alloc(sizeof(int2) * op.rows * (size_t)op.steps);
-        unsigned char *glen = (unsigned char *)dev_alloc((op.rows + 31) / 32);
-        mem.push_back(tap);
-        mem.push_back(glen);
-        k_row_taps<<<setup_blocks(op.rows), kSB, 0, s>>>(P.L[l], C, ring, op.rows, op.steps, tap, glen);
+        at[l].tap = second.take(sizeof(int2) * op.rows * (size_t)op.steps);
+        at[l].glen = second.take((op.rows + 31) / 32);
+    }
+    if (G == 0) return;
+    unsigned char *const rows = (unsigned char *)dev_alloc(second.bytes);
+    mem.push_back(rows);
+    for (int l = 0; l < G; l++) {
+        const StencilDev &C = P.L[l + 1].S;
+        const int ring = host.irregular[l] == 0;
+        SparseOp &op = out->rst[l];
+        int2 *tap = (int2 *)(rows + at[l].tap);
+        k_row_taps<<<setup_blocks(op.rows), kSB, 0, s>>>(P.L[l], C, ring, op.rows, op.steps, tap, rows + at[l].glen);
         GGB_LAUNCHED();
         op.tap = tap;
-        op.glen = glen;
+        op.glen = rows + at[l].glen;
         if (ring) {
-            float *rw16 = (float *)dev_alloc(sizeof(float) * 16 * (size_t)C.n);
-            mem.push_back(rw16);
+            float *rw16 = (float *)(vectors + at[l].rw16);
             k_build_rw16<<<setup_blocks(C.n), kSB, 0, s>>>(P.L[l], C, rw16);
             GGB_LAUNCHED();
             out->rw16[l] = rw16;
         }
-        out->r[l] = dev_alloc(sizeof(float) * (size_t)P.L[l].S.n);
-        out->b[l + 1] = dev_alloc(sizeof(float) * (size_t)(C.n + 8));
-        out->xo[l + 1] = dev_alloc(sizeof(float) * (size_t)(C.n + 8));
-        for (void *p : {out->r[l], out->b[l + 1], out->xo[l + 1]}) mem.push_back(p);
     }
-    GGB_CHECK(cudaStreamSynchronize(s));
-    dev_free(scratch);
 }
 
 // The mixed solve's: the same transfers, FP16 level vectors, and below level 0
@@ -224,7 +257,11 @@ void levels_build_mixed(const SolveParams &P, const LevelSet &plain, LevelSet *o
     for (int l = 0; l < P.nlev_grid; l++) {
         const StencilDev &S = P.L[l].S, &C = P.L[l + 1].S;
         if (l > 0) {
-            ring_links(S, 1, out, l, mem, bad);
+            int2 *link = (int2 *)dev_alloc(ring_link_bytes(S));
+            int *cell = (int *)dev_alloc(ring_cell_bytes(S));
+            mem.push_back(link);
+            mem.push_back(cell);
+            ring_links(S, 1, link, cell, out, l, bad);
             float *w = (float *)dev_alloc(sizeof(float) * 4 * (size_t)S.wplane);
             mem.push_back(w);
             k_round_half<<<setup_blocks(4 * (size_t)S.wplane), kSB, 0, stream()>>>(4 * (size_t)S.wplane, S.wpad, w);
