@@ -44,9 +44,10 @@
 
 namespace ggb {
 
-namespace {
+namespace pcg_setup {
 #include "solver_body.cuh"
 }
+using namespace pcg_setup;
 
 // solver_plain.cu, solver_plain_sweeps.cu, solver_mixed.cu, solver_mixed_sweeps.cu
 const void *pcg_kernel_plain(int threads, bool batch);

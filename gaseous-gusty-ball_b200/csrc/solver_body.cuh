@@ -1,6 +1,6 @@
 // solver_body.cuh — the device code of the persistent solve kernels k_pcg /
-// k_pcg_batch (constants, stencil phases, V-cycle, PCG body), included inside an
-// unnamed namespace by solver.cu (set-up kernels and the host side) and by
+// k_pcg_batch (constants, stencil phases, V-cycle, PCG body), included inside a
+// namespace of its own by solver.cu (set-up kernels and the host side) and by
 // solver_{plain,mixed}{,_sweeps}.cu, which compile the solve kernels of one
 // precision and coarse end each: a module is brought to the device as a whole, and
 // all 24 kernels in one cost a program's first call 18 ms.
@@ -13,10 +13,10 @@
 // inlined once, in loops over levels and iterations (a variant with 640 KB of code
 // spent a seventh of its stall cycles on instruction fetch), no static operand is
 // read between a barrier and the values that wait for it, and the window of a
-// phase holds FP32 values only.  Solve in ms, before (values, four FP64 weights
-// and three inputs of every window cell staged anew in each phase) and after:
-// N = 64 0.273, 0.230; N = 256 0.869, 0.757; N = 512 2.33, 1.92; mixed 0.852,
-// 0.757 and 2.23, 1.89.  The FP32 and FP16 roundings of every vector are unchanged.
+// phase holds FP32 values only.  A step's solve in ms, before (values, four FP64
+// weights and three inputs of every window cell staged anew in each phase) and now:
+// N = 256 0.869, 0.701; N = 512 2.33, 1.84, mixed 2.23, 1.79; a cold solve to 1e-6:
+// N = 64 0.459, 0.324.  The FP32 and FP16 roundings of every vector are unchanged.
 
 constexpr int kPBNarrow = 384;   // threads per block of the persistent kernel on small grids
 constexpr int kPB = 512;         // ... on ordinary ones
@@ -24,11 +24,11 @@ constexpr int kPBWide = 1024;     // ... where the fine levels' bytes outweigh t
 // Cells per block up to which blocks are narrow: with few cells a thread, a
 // phase's time is its barrier and the issue of the warps' common part (sums,
 // index arithmetic, block barriers), of which 12 warps have less than 16.  512 /
-// 384 threads on 148 SMs, ms: N = 32 0.178 / 0.169, 64 0.241 / 0.230, 128 0.495 /
-// 0.477, 192 0.626 / 0.622, 256 (2657 cells) 0.759 / 0.758, 384 1.25 / 1.34; 256
-// and 320 threads are slower from N = 128 on (0.522, 0.504).
+// 384 threads on 148 SMs, cold solves to 1e-6 in ms: N = 32 0.241 / 0.223, 64 0.348
+// / 0.324, 128 0.543 / 0.518, 192 0.704 / 0.687, 256 (2657 cells) 0.840 / 0.824, 288
+// 1.076 / 1.075, 384 1.56 / 1.66; 256 and 320 threads were slower from N = 128 on.
 constexpr int kNarrowCells = 2700;
-constexpr int kWideMinN = 480;    // 512 / 1024 threads, ms: N = 448 1.57 / 1.68, 512 1.97 / 1.92
+constexpr int kWideMinN = 480;    // 512 / 1024 threads, the same, ms: N = 448 1.99 / 2.05, 480 2.48 / 2.52, 512 2.54 / 2.47
 // Cells a thread takes at once in the vector updates of a solve without multigrid:
 // the loads of all before the stores of any, which the compiler cannot tell apart.
 // 100 iterations in us, one cell / 3: N = 64 786 / 722, 256 2031 / 1381, 512 4680 /
@@ -153,7 +153,7 @@ __device__ __noinline__ void trace_mark(SolveTrace *t, unsigned long long mark) 
 // polling every other's slot, measured 4 us a barrier against 1.7 + 1.2.)
 // A row's values are asked for together (a lane of a 148-block solve has four or
 // five; in a loop with a remainder they come one L2 round trip after the other),
-// and those of both sums at once: 2.1 us a barrier before, 0.7 now.
+// and those of both sums at once: a barrier with sums took 4.3 us, now 2.2.
 constexpr int kRowLoads = 5;
 template <int NV>
 __device__ __forceinline__ void rows_total(const double *row, int nb, int lane, double (&v)[NV]) {

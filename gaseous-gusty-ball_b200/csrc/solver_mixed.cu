@@ -5,10 +5,10 @@
 
 namespace ggb {
 
-namespace {
+namespace pcg_mixed {
 #include "solver_body.cuh"
 }
 
-const void *pcg_kernel_mixed(int threads, bool batch) { return kernel_of<true, false>(threads, batch); }
+const void *pcg_kernel_mixed(int threads, bool batch) { return pcg_mixed::kernel_of<true, false>(threads, batch); }
 
 }  // namespace ggb

@@ -4,10 +4,10 @@
 
 namespace ggb {
 
-namespace {
+namespace pcg_mixed_sweeps {
 #include "solver_body.cuh"
 }
 
-const void *pcg_kernel_mixed_sweeps(int threads, bool batch) { return kernel_of<true, true>(threads, batch); }
+const void *pcg_kernel_mixed_sweeps(int threads, bool batch) { return pcg_mixed_sweeps::kernel_of<true, true>(threads, batch); }
 
 }  // namespace ggb

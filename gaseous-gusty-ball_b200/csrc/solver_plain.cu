@@ -5,10 +5,10 @@
 
 namespace ggb {
 
-namespace {
+namespace pcg_plain {
 #include "solver_body.cuh"
 }
 
-const void *pcg_kernel_plain(int threads, bool batch) { return kernel_of<false, false>(threads, batch); }
+const void *pcg_kernel_plain(int threads, bool batch) { return pcg_plain::kernel_of<false, false>(threads, batch); }
 
 }  // namespace ggb

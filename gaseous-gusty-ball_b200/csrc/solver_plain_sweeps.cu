@@ -4,10 +4,10 @@
 
 namespace ggb {
 
-namespace {
+namespace pcg_plain_sweeps {
 #include "solver_body.cuh"
 }
 
-const void *pcg_kernel_plain_sweeps(int threads, bool batch) { return kernel_of<false, true>(threads, batch); }
+const void *pcg_kernel_plain_sweeps(int threads, bool batch) { return pcg_plain_sweeps::kernel_of<false, true>(threads, batch); }
 
 }  // namespace ggb
