@@ -361,6 +361,8 @@ __device__ __forceinline__ void stencil_phase(int l, RingPre &R, Load load, Cell
     const int total = 48 * S.nring, stride = 32 * vwarps();
 #pragma unroll 1
     for (int e0 = 32 * vwarp(); e0 < total; e0 += stride) {
+        RingPre next = R;  // the next links beside this round's values: few blocks take many rounds
+        if (e0 + stride < total) ring_load(L, min(e0 + stride + lane, total - 1), next);
         const int c = R.own & 0xffffff;
         const float xo = load(c), xn = load(R.q.x);
         const A d = (A)xo - (A)xn, w = (A)__int_as_float(R.q.y);
@@ -390,7 +392,7 @@ __device__ __forceinline__ void stencil_phase(int l, RingPre &R, Load load, Cell
             for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         }
         if (e0 + lane < total && (lane & 7) == 0) cell(c, xo, v);
-        if (e0 + stride < total) ring_load(L, min(e0 + stride + lane, total - 1), R);
+        R = next;
     }
     float *win = s_win();
 #pragma unroll 1
