@@ -1,6 +1,6 @@
 """Poisson solves over the forms of the multigrid hierarchy's coarse end: one
-level only, a coarsest level held as a dense map (up to 32 cells an edge),
-and a larger one that is swept.
+level only (swept), a coarsest level held as a dense map (up to 16 cells an
+edge), and a larger one that is swept.
 
 Against the FP64 oracle on the same tables, solved to a relative residual of
 1e-10.  The solve here stops at 1e-6; the oracle's psi then differs by the
