@@ -116,11 +116,11 @@ static int pcg_threads(const SolveParams &p) {
 // since few blocks have many of them: by cells alone, 45 planets of N = 32 (1870 a
 // block, 467 rows) and 6 of N = 100 (2430, no rows) would count as equals.  Batched
 // solves in us with 384 / 512 / 1024 threads, by work per block:
-//   2 planets of N = 64, 540: 323 336 453; 4 of 64, 1080: 375 383 502
-//   10 of N = 32, 1450: 403 350 489; 6 of 64, 1620: 491 437 585; 2 of 128, 1540: 517 547 673
-//   12 of 64, 3240: 843 720 755; 5 of 128, 3840: 972 880 943; 6 of 100, 5470: 2472 2372 2670
-//   2 of 256, 5520: 1187 1136 1222; 8 of 128, 6140: 1324 1187 1200; 24 of 64, 6480: 1468 1219 1146
-//   45 of 32, 6540: 1470 1210 1107; 20 of 25, 10600: 4185 4324 1815; 148 of 32, 21500: 4012 3318 2819
+//   2 planets of N = 64, 540: 311 327 434; 4 of 64, 1080: 364 374 473
+//   10 of N = 32, 1450: 385 343 443; 6 of 64, 1620: 436 409 533; 2 of 128, 1540: 493 525 631
+//   12 of 64, 3240: 758 665 682; 5 of 128, 3840: 889 814 881; 6 of 100, 5470: 2534 2461 2465
+//   2 of 256, 5520: 1155 1109 1181; 8 of 128, 6140: 1246 1132 1126; 24 of 64, 6480: 1313 1128 1033
+//   45 of 32, 6540: 1263 1098 946; 20 of 25, 10600: 4184 4067 1762; 148 of 32, 21500: 3415 2995 2437
 // One planet on the whole launch has fluid_step's choice (and so its sums).
 constexpr int kDenseWork = 10, kSweepWork = 20;
 constexpr int kNarrowWork = 1100, kWideWork = 5800;

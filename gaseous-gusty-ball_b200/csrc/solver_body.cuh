@@ -627,10 +627,13 @@ __device__ __forceinline__ void vcycle_block_smem(const SolveParams &P, int l0, 
 // reduction and two block barriers, and convert b anew: from three rounds on
 // (BATCH) b goes to shared memory once as FP64 and every warp takes whole rows.
 // Same sums.  Batched solves in us, rounds / rows: 12 planets of N = 64 (512 threads)
-// 894 / 720; 24 of N = 64 (1024) 1292 / 1146; 60 of N = 32 2028 / 1507, 148 3924 /
-// 2819.  4 of N = 64 (384): whole rows from nine rounds on 405, from three 375.  (In
-// the kernels of single solves the rows' registers cost N = 512 1.5 %.)
+// 894 / 665; 24 of N = 64 (1024) 1292 / 1033; 60 of N = 32 2028 / 1267, 148 3924 /
+// 2437; with a loop over a row's loads instead of kRowAhead asked for together (a
+// remainder goes one L2 round trip at a time) 689, 1116, 1490 and 2789, and 148 of N =
+// 16 647 where it is 531.  4 of N = 64 (384): whole rows from nine rounds on 405, from
+// three 375.  (In the kernels of single solves the rows' registers cost N = 512 1.5 %.)
 constexpr int kDensePre = 6;
+constexpr int kRowAhead = 3;  // 16-byte loads of either half of a row in flight (BATCH)
 struct DenseTaps {
     float4 w[kDensePre];
 };
@@ -668,12 +671,21 @@ __device__ __forceinline__ void dense_rows(const DenseTaps &T, Get4 get4, Put pu
                 v += (double)w.z * q.x;
                 v += (double)w.w * q.y;
             };
-#pragma unroll 3
-            for (int j = lane; j < h4; j += 32) {
-                const int k = min(j + h4, ld4 - 1);
-                const float4 w0 = __ldg(d + j), w1 = __ldg(d + k);
-                add(v0, w0, j);
-                if (j + h4 < ld4) add(v1, w1, k);
+#pragma unroll 1
+            for (int jb = lane; jb - lane < h4; jb += 32 * kRowAhead) {
+                float4 w0[kRowAhead], w1[kRowAhead];
+#pragma unroll
+                for (int u = 0; u < kRowAhead; u++) {
+                    const int j = min(jb + 32 * u, h4 - 1);
+                    w0[u] = __ldg(d + j);
+                    w1[u] = __ldg(d + min(j + h4, ld4 - 1));
+                }
+#pragma unroll
+                for (int u = 0; u < kRowAhead; u++) {
+                    const int j = jb + 32 * u;
+                    if (j < h4) add(v0, w0[u], j);
+                    if (j < h4 && j + h4 < ld4) add(v1, w1[u], j + h4);
+                }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
